@@ -181,7 +181,7 @@ constexpr int kDpCandidates = 2;
 constexpr int kScoreRowsCand[kScoreCandidates] = {16, 8, 32, 16, 16};
 constexpr int kWindowCand[kScoreCandidates] = {1024, 1024, 1024, 256, 4096};
 constexpr int kDpWarpsCand[kDpCandidates] = {2, 1};
-constexpr int kPreferredScoreCand = 2;     // 32 rows, window 1,024
+constexpr int kPreferredScoreCand = 0;     // 16 rows, window 1,024
 constexpr float kTuneMargin = 0.015f;      // a candidate must be this much faster to replace it
 struct Tuning {
     int rows = 16, window = kOrderWindow, dp_warps = 2;
@@ -579,9 +579,11 @@ void tune_kernels(cbp_context* c, const ScoreArgs& base, int p0, int p1, Tuning&
         if (t.score_ms[k] < t.score_ms[bs]) bs = k;
     }
     // The candidates' sample times lie within about 1 % of each other, the
-    // sample's noise. Unless one is clearly faster, keep 32 rows per block
-    // with the default window: the fewest re-reads of the database lists,
-    // and the fastest on full-size slabs.
+    // sample's noise. Unless one is clearly faster, keep 16 rows per block
+    // with the default window: 8 blocks fit an SM as with 8 rows (5 with 32,
+    // whose query lists take 42 KB), with half the re-reads of the database
+    // lists. q400 x 1,000 profiles: 77.4 ms with 8 rows, 78.0 with 16, and 82
+    // with 32.
     if (t.score_ms[bs] > (1.0f - kTuneMargin) * t.score_ms[kPreferredScoreCand]) bs = kPreferredScoreCand;
     Dp1Args d;
     d.scores = a.scores;

@@ -11,11 +11,11 @@
 //
 // DDMS dominates the cost (~550 segment-DP steps per cell for 99-distance
 // lists); it is CUDA-core ALU-bound, so the kernel is shaped for issue
-// efficiency: byte-packed distance lists brought in by bulk copies and kept
-// in shared memory at an odd word stride (conflict-free for lanes in step),
-// a 22x22 pair-score table in shared memory, one code path for upper and
-// lower diagonals, and the step loop unrolled by four with DSTSEGM as
-// compile-time cases.
+// efficiency: distance lists split by parity in shared memory, the database's
+// as bytes at an odd word stride (conflict-free for lanes in step), a word of
+// four read at once and byte and table row combined by one dp4a; a 22x22
+// pair-score table in shared memory; the segment register reached only by
+// steps that can change it; and DSTSEGM as compile-time cases.
 #include <cmath>
 #include "cother_b200.h"
 #include "common.cuh"
@@ -31,64 +31,35 @@ namespace {
 constexpr int kCols = 32;          // database positions per block (one per lane)
 constexpr int kWarps = 4;
 constexpr int kThreads = kCols * kWarps;
-constexpr int kElems = 104;        // list elements held per position (99 + overrun)
-constexpr int kDbStride = 108;     // bytes per database list in shared memory (27 words)
 constexpr int kDbCopy = 112;       // bytes of a list brought in by one bulk copy (and its packed stride)
-constexpr int kDbWords = kDbStride / 4;
+// The diagonals of the DDMS step through the lists two elements at a time,
+// so a diagonal reads elements of one parity only: a database list is kept
+// as its even and its odd elements, bytes, element m of a parity at byte
+// m + 3 of its kHalfWords words (element 1 starts a word).
+constexpr int kHalfWords = 16;
+constexpr int kDbWords = 2 * kHalfWords + 1;   // an odd stride: lanes in step do not conflict
+// A query list is kept as 32-bit byte offsets into the pair-score table
+// (code x 88): the even elements for the upper diagonals, element m at word
+// m + 3 (element 1 on 16 bytes), and for the lower diagonals the elements of
+// the parity they use twice, element n at word n + 1 and at word n, so that
+// element n0 + 1 starts on 8 bytes for even and for odd n0.
+constexpr int kQUp = 64, kQLow = 60;
+constexpr int kQWords = kQUp + 2 * kQLow;
 constexpr unsigned long long kListWaitNs = 1000000000ull;   // the lists' copies: a wait gives up after 1 s
 
 // Top-3 register of non-intersecting segments
 // (src/libmycu/cusco/CuBatchScoreMatrix_ddms2s.cuh:182-251). The reference
 // packs a segment's coordinates into one word [QB QE PB PE] and tests
 // intersection with per-byte SIMD min/max. Here a segment is two words,
-// begins (QB<<16 | PB) and ends (QE<<16 | PE), so that the test uses the
-// native halfword SIMD min/max of sm_90+: two segments intersect when their
-// query OR their database ranges overlap (ddms2s.cuh:162-173), i.e. when
-// min(end) >= max(begin) in either halfword; adding 256 to each halfword
-// before subtracting keeps both non-negative (positions < 256), so the test
-// is whether bits 8..15 of either half are set. The coordinates of an empty
-// entry (score 0) are never consulted for a decision, as in the reference.
-__device__ __forceinline__ uint32_t vmax_u16x2(uint32_t a, uint32_t b)
-{
-    uint32_t r;
-    asm("max.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-    return r;
-}
-__device__ __forceinline__ uint32_t vmin_u16x2(uint32_t a, uint32_t b)
-{
-    uint32_t r;
-    asm("min.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-    return r;
-}
+// begins (QB<<16 | PB) and ends (QE<<16 | PE), the ends with the top bit of
+// each halfword set: two segments intersect when their query OR their
+// database ranges overlap (ddms2s.cuh:162-173), i.e. when in either halfword
+// both ends are at or past the other's begin, and with the guard bits each
+// difference keeps its top bit exactly then (positions < 32768).
+constexpr uint32_t kGuard = 0x80008000u;
 __device__ __forceinline__ bool seg_intersect(uint32_t b1, uint32_t e1, uint32_t b2, uint32_t e2)
 {
-    const uint32_t mx = vmax_u16x2(b1, b2), mn = vmin_u16x2(e1, e2);
-    return ((mn + 0x01000100u - mx) & 0xff00ff00u) != 0u;
-}
-// The update proper, for a candidate s >= ms[2] whose intersection with the
-// top entry (x0) is known and that changes the register: s >= ms[0] or not
-// x0. Every case of the reference's register tests the candidate against
-// the entries at ranks 0 and 1 (an empty entry's test never matters).
-__device__ __forceinline__ void register_max(float (&ms)[3], uint32_t (&mb)[3], uint32_t (&me)[3],
-                                             float s, uint32_t cb, uint32_t ce, bool x0)
-{
-    const bool x1 = seg_intersect(cb, ce, mb[1], me[1]);
-    if (ms[0] <= s) {
-        const float a1 = x0 ? 0.0f : ms[0];
-        const float a2 = x1 ? 0.0f : ms[1];
-        const bool up = (a1 == 0.0f);
-        ms[2] = up ? 0.0f : a2;
-        ms[1] = up ? a2 : a1;
-        const uint32_t b1 = up ? mb[1] : mb[0], e1 = up ? me[1] : me[0];
-        mb[2] = mb[1]; me[2] = me[1];
-        mb[1] = b1; me[1] = e1;
-        ms[0] = s; mb[0] = cb; me[0] = ce;
-    } else if (ms[1] <= s) {          // not x0 here
-        ms[2] = x1 ? 0.0f : ms[1]; mb[2] = mb[1]; me[2] = me[1];
-        ms[1] = s; mb[1] = cb; me[1] = ce;
-    } else if (!x1) {                 // ms[2] <= s, not x0
-        ms[2] = s; mb[2] = cb; me[2] = ce;
-    }
+    return ((e1 - b2) & (e2 - b1) & kGuard) != 0u;
 }
 
 // Saturating add/multiply: the result clamped to [0, 1] in one FMA-pipe
@@ -99,12 +70,6 @@ __device__ __forceinline__ float sat_add(float a, float b)
     asm("add.sat.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
     return r;
 }
-__device__ __forceinline__ float sat_mul(float a, float b)
-{
-    float r;
-    asm("mul.sat.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
-    return r;
-}
 __device__ __forceinline__ float sat_fma(float a, float b, float c)
 {
     float r;
@@ -112,15 +77,100 @@ __device__ __forceinline__ float sat_fma(float a, float b, float c)
     return r;
 }
 
-// smallest positive float: the register filter's threshold while its third
-// entry is empty (every positive candidate is at least this)
+// The third score while its entry is empty: the smallest positive float, so
+// that it is also the register's threshold (every positive candidate is at
+// least this).
 constexpr float kTiny = 0x1p-149f;
+constexpr unsigned kFull = 0xffffffffu;
+
+// The register of one cell: the three scores in order, and the coordinates
+// of the first two entries (every change of the register drops the third,
+// so its coordinates are never consulted; nor are an empty entry's).
+struct DdmsReg {
+    float m0 = 0.0f, m1 = 0.0f, m2 = kTiny;
+    uint32_t b0 = 0, e0 = kGuard, b1 = 0, e1 = kGuard;
+};
+
+// Lengths are kept in units of 2^22, as the bits of a float: see
+// ddms_diagonal().
+constexpr int kLenUnit = 1 << 22;
+
+// The bits of a length, as a float, grow with it, so a saturating multiply-add
+// turns them into 1 at DSTSEGM - 1 units and above and 0 below.
+struct LenMask { float scale, bias; };
+template <int kSeg>
+__device__ __forceinline__ LenMask len_mask(int dst)
+{
+    if (kSeg == 6) return {0x1p126f, -2.0f};       // 5 units: 1.5 x 2^-125; 4 units: 2^-125
+    if (dst == 1) return {0.0f, 1.0f};
+    const float at = __int_as_float((dst - 1) * kLenUnit), below = __int_as_float((dst - 2) * kLenUnit);
+    const float scale = __fdiv_rn(1.0f, at - below);   // a power of two, at most 2^127
+    return {scale, -(below * scale)};
+}
+
+// The best candidate of one 4-step, offered to the register: t1..t4 are the
+// running sums after the step's elements, c0..c3 the elements since the sum
+// was last zero, up to the element before each (a candidate needs DSTSEGM - 1
+// of them), pos the query and database index of the step's first element. All
+// three cases of the reference's register are one rule: a candidate at or
+// above the third score enters unless it intersects an entry of a higher
+// score; entering, it removes the entries of at most its score that it
+// intersects, and the third.
+//
+// Returns the threshold of the lane until the running segment ends: a later
+// candidate of the same segment has the same begin and a larger end, so it
+// intersects what this one does, and below this one's score (if it entered)
+// or below that of the entry that rejected it, it changes nothing. Without
+// that threshold a lane of 57 % of the warp steps has a candidate at or above
+// its third entry; with it, 36 % (a CPU emulation of the warps on the lists of
+// a 400-position query and 200 profiles).
+template <int kSeg>
+__device__ __forceinline__ float ddms_offer(DdmsReg& r, bool on, uint32_t pos, float thr, LenMask lm, int c0, int c1,
+                                            int c2, int c3, float t1, float t2, float t3, float t4)
+{
+    // the sum where the segment is long enough, else 0
+    const float v1 = t1 * sat_fma(__int_as_float(c0), lm.scale, lm.bias);
+    const float v2 = t2 * sat_fma(__int_as_float(c1), lm.scale, lm.bias);
+    const float v3 = t3 * sat_fma(__int_as_float(c2), lm.scale, lm.bias);
+    const float v4 = t4 * sat_fma(__int_as_float(c3), lm.scale, lm.bias);
+    const float s = fmaxf(fmaxf(v1, v2), fmaxf(v3, v4));
+    const bool ok = on & (thr <= s);
+    if (ok) {
+        // ending at the first element that attains it
+        const uint32_t k = (v1 == s) ? 0x80018001u : (v2 == s) ? 0x80028002u : (v3 == s) ? 0x80038003u : 0x80048004u;
+        const uint32_t ce = pos + k;
+        // DSTSEGM >= 5: the candidate, at least 5 long and ending at most 4
+        // past the step's first element, contains it: c0 elements up to it
+        uint32_t cb;
+        if (kSeg != 1) {
+            cb = (pos + 0x00010001u) - __umulhi((uint32_t)c0, 0x00010001u << 10);
+        } else {
+            const int ck = (v1 == s) ? c0 : (v2 == s) ? c1 : (v3 == s) ? c2 : c3;
+            cb = (ce - kGuard) - __umulhi((uint32_t)ck, 0x00010001u << 10);
+        }
+        const bool x0 = seg_intersect(cb, ce, r.b0, r.e0);
+        const bool x1 = seg_intersect(cb, ce, r.b1, r.e1);
+        const bool g0 = r.m0 <= s, g1 = r.m1 <= s;
+        const bool rej0 = x0 & !g0, rej1 = x1 & !g1;
+        thr = rej0 ? r.m0 : rej1 ? r.m1 : s;
+        if (!rej0 & !rej1) {
+            if (x1) r.m1 = 0.0f;
+            r.m2 = fmaxf(g1 ? r.m1 : s, kTiny);
+            if (g0) {
+                if (x0) r.m2 = kTiny;
+                else { r.m1 = r.m0; r.b1 = r.b0; r.e1 = r.e0; }
+                r.m0 = s; r.b0 = cb; r.e0 = ce;
+            } else if (g1) {
+                r.m1 = s; r.b1 = cb; r.e1 = ce;
+            }
+        }
+    }
+    return thr;
+}
 
 // One diagonal of the DDMS segment DP. Elements e = 0,1,... pair query list
 // element oq+e with database list element od+e (upper diagonals: oq = 0,
-// od = j; lower: oq = i, od = 0). The lists hold their codes pre-multiplied
-// into byte offsets of the pair-score table T (query: code x 88, a row of
-// 22 floats; database: code x 4), so a pair score is one add and one load. Pair scores at even offsets within each
+// od = j; lower: oq = i, od = 0). Pair scores at even offsets within each
 // 4-step are table values, odd ones the mean of their neighbours
 // (src/libmycu/cusco/CuBatchScoreMatrix_ddms2s_h2.cuh:184-198); a segment
 // restarts when the running sum has fallen to zero, and the best segment of
@@ -131,108 +181,116 @@ constexpr float kTiny = 0x1p-149f;
 // [0, 1) and max(sum, 0) is one saturating add; scaling by a power of two
 // commutes exactly with IEEE rounding, so the sums are the reference's
 // times 2^-7, bit for bit. An odd element's mean 0.5*(a+b) is exact once a+b
-// is rounded, so adding it is one saturating fma(0.5, a+b, sum). The segment length is a small exact float:
-// len_k = len_{k-1} * [sum_{k-1} > 0] + 1, the indicator being
-// sat(sum * 2^100) (every positive sum here is far above 2^-100). A step's
-// candidate is max_k sum_k * [len_k >= DSTSEGM] and sits at the first k that
-// attains it, which is the reference's strict "<" scan. `thr` is
-// max(third entry's score, kTiny): a candidate below it changes nothing.
-// kLongSegments: DSTSEGM >= 5 (the default is 6), a compile-time case so
-// that the candidate's begin needs no run-time test in the step loop
-// (measured 1.9 % faster than the uniform branch).
-template <bool kLongSegments>
+// is rounded, so adding it is one saturating fma(0.5, a+b, sum). The bits of
+// a sum, as an integer, are 0 when it is zero and above 105 x 2^22 (the bits
+// of 2^-75) when not: the table's values are multiples of 2^-56, and so is
+// every sum of them. So the number of elements since the last zero, in units
+// of 2^22, is min(c + 2^22, bits), one instruction (VIADDMNMX) for the two
+// that a float length needs.
+//
+// A step can offer a candidate (DSTSEGM >= 5) only when its first sum is
+// positive and c1 >= DSTSEGM - 3, which is all that every step tests; the
+// masked sums and the register are in ddms_offer(), in 64 % and 36 % of the
+// warp steps. What bounds the kernel is instruction issue (0.87 a cycle and
+// scheduler), with the ALU pipe, which takes an instruction every other
+// cycle, at 69 %: the steps' arithmetic is therefore spread over both pipes
+// (sums and masks FMA, lengths ALU, table offsets the FMA pipe's dp4a).
+// Measured at q400 x 1,000 profiles: 51.0 warp instructions a step and 77.4
+// ms, against 59.2 and 85.8 ms with float lengths, the masked sums in every
+// step and no threshold per segment; with the masks in every step 82 ms, with
+// a running maximum tested first 86 ms, with votes for the branches 91 ms.
+//
+// qw: words of elements 1.. of the query list on this diagonal, q0 its
+// element 0; dw, sel: the words that hold elements 1.. of the database list
+// (upper: the byte selector that aligns them), d0 its element 0; ks: the
+// multipliers that pick byte 0..3 of a word and scale it to a table offset.
+template <bool kUpper, int kSeg>
 __device__ __forceinline__ void ddms_diagonal(
-    const uint16_t* __restrict__ q, const uint8_t* __restrict__ d,
-    const char* __restrict__ T, int lim, int oq, int od, float nsegm1,
-    float (&ms)[3], uint32_t (&mb)[3], uint32_t (&me)[3], float& thr)
+    const uint32_t* __restrict__ qw, uint32_t q0, const uint32_t* __restrict__ dw, uint32_t sel, uint32_t d0,
+    const char* __restrict__ T, int lim, uint32_t pos0, int dst, LenMask lm, uint4 ks, DdmsReg& r)
 {
-    constexpr float kBig = 0x1p100f;
-    float s0 = *reinterpret_cast<const float*>(T + q[0] + d[0]);
+    const int need = (kSeg == 6 ? 5 : dst - 1) * kLenUnit;
+    float s0 = *reinterpret_cast<const float*>(T + (q0 + 4u * d0));
     float t = sat_add(s0, 0.0f);
-    float ls = 1.0f;
-    const uint32_t cbase = ((uint32_t)oq << 16) | (uint32_t)od;
-    // four steps per iteration (measured: 2.2 % faster than the compiler's
-    // own choice, 3.6 % slower with two, 12 % slower with eight)
-#pragma unroll 4
-    for (int x = 0; x < lim; x += 4) {
-        const float s2 = *reinterpret_cast<const float*>(T + q[x + 2] + d[x + 2]);
-        const float s4 = *reinterpret_cast<const float*>(T + q[x + 4] + d[x + 4]);
-        const float l1 = __fmaf_rn(ls, sat_mul(t, kBig), 1.0f);
+    int c = t > 0.0f ? kLenUnit : 0;
+    float thr = 0.0f;
+    uint32_t cur = dw[0];
+    auto step = [&](float s2, float s4, int x, bool on) {
         const float t1 = sat_fma(0.5f, s0 + s2, t);
-        const float l2 = __fmaf_rn(l1, sat_mul(t1, kBig), 1.0f);
+        const int c1 = __viaddmin_s32(c, kLenUnit, __float_as_int(t1));
         const float t2 = sat_add(t1, s2);
-        const float l3 = __fmaf_rn(l2, sat_mul(t2, kBig), 1.0f);
+        const int c2 = __viaddmin_s32(c1, kLenUnit, __float_as_int(t2));
         const float t3 = sat_fma(0.5f, s2 + s4, t2);
-        const float l4 = __fmaf_rn(l3, sat_mul(t3, kBig), 1.0f);
+        const int c3 = __viaddmin_s32(c2, kLenUnit, __float_as_int(t3));
         const float t4 = sat_add(t3, s4);
-        const float v1 = t1 * sat_add(l1, nsegm1);
-        const float v2 = t2 * sat_add(l2, nsegm1);
-        const float v3 = t3 * sat_add(l3, nsegm1);
-        const float v4 = t4 * sat_add(l4, nsegm1);
-        const float scom = fmaxf(fmaxf(v1, v2), fmaxf(v3, v4));
-        // the register is sorted by score, so a candidate below its third
-        // entry changes nothing (every branch of register_max fails)
-        if (thr <= scom) {
-            const int k = (v1 == scom) ? 1 : (v2 == scom) ? 2 : (v3 == scom) ? 3 : 4;
-            const uint32_t be = (uint32_t)(x + k);
-            uint32_t bb;
-            if (kLongSegments) {
-                // DSTSEGM >= 5: the candidate, at least 5 long and ending at
-                // x+k <= x+4, contains element x, so it is the segment running
-                // at x, which began at x + 1 - ls
-                bb = (uint32_t)(x + 1) - (uint32_t)ls;
-            } else {
-                const float lk = (v1 == scom) ? l1 : (v2 == scom) ? l2 : (v3 == scom) ? l3 : l4;
-                bb = be + 1u - (uint32_t)lk;
-            }
-            const uint32_t cb = cbase + bb * 0x00010001u, ce = cbase + be * 0x00010001u;
-            // below the top entry and intersecting it, a candidate changes
-            // nothing (the reference's second and third cases both require
-            // no intersection with the top); most candidates end here
-            const bool x0 = seg_intersect(cb, ce, mb[0], me[0]);
-            if (ms[0] <= scom || !x0) {
-                register_max(ms, mb, me, scom, cb, ce, x0);
-                thr = fmaxf(ms[2], kTiny);
-            }
+        const uint32_t pos = pos0 + (uint32_t)x * 0x00010001u;
+        if (kSeg != 1) {
+            // a segment's first step that can offer has c1 <= DSTSEGM units:
+            // its threshold is the register's
+            const bool fresh = c1 <= need + kLenUnit;
+            if (c1 >= need - 2 * kLenUnit)
+                thr = ddms_offer<kSeg>(r, on, pos, fresh ? r.m2 : thr, lm, c, c1, c2, c3, t1, t2, t3, t4);
+        } else {
+            (void)ddms_offer<kSeg>(r, on, pos, r.m2, lm, c, c1, c2, c3, t1, t2, t3, t4);
         }
         s0 = s4;
         t = t4;
-        ls = l4;
+        c = __viaddmin_s32(c3, kLenUnit, __float_as_int(t4));
+    };
+    auto score = [&](uint32_t o) { return *reinterpret_cast<const float*>(T + o); };
+    // two steps an iteration: four elements of each list (unrolled further,
+    // or with the scores of the next iteration fetched ahead, it was slower)
+#pragma unroll 1
+    for (int x = 0; x < lim; x += 8) {
+        uint32_t d, o0, o1, o2, o3;
+        if (kUpper) {
+            const uint32_t nxt = dw[(x >> 3) + 1];
+            d = __byte_perm(cur, nxt, sel);
+            cur = nxt;
+            const uint4 o = *reinterpret_cast<const uint4*>(qw + (x >> 1));
+            o0 = o.x; o1 = o.y; o2 = o.z; o3 = o.w;
+        } else {
+            d = dw[x >> 3];
+            const uint2 a = *reinterpret_cast<const uint2*>(qw + (x >> 1));
+            const uint2 b = *reinterpret_cast<const uint2*>(qw + (x >> 1) + 2);
+            o0 = a.x; o1 = a.y; o2 = b.x; o3 = b.y;
+        }
+        const float sa = score(__dp4a(d, ks.x, o0)), sb = score(__dp4a(d, ks.y, o1));
+        const float sc = score(__dp4a(d, ks.z, o2)), sd = score(__dp4a(d, ks.w, o3));
+        step(sa, sb, x, true);
+        step(sc, sd, x + 4, x + 4 < lim);
     }
 }
 
 // DDMS of one cell (src/libmycu/cusco/CuBatchScoreMatrix_ddms2s_h2.cuh:433-500).
 // Returns the top-3 sum in the reference's scale.
-__device__ __forceinline__ float ddms_cell(const uint16_t* __restrict__ q, int len1,
-                                           const uint8_t* __restrict__ d, int len2,
-                                           const char* __restrict__ T, int dstsegm)
+template <int kSeg>
+__device__ __forceinline__ float ddms_cell(const uint32_t* __restrict__ q, int len1,
+                                           const uint32_t* __restrict__ d, int len2,
+                                           const char* __restrict__ T, int dst, uint4 ks)
 {
-    float ms[3] = {0.0f, 0.0f, 0.0f};
-    uint32_t mb[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu};
-    uint32_t me[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu};
-    const float nsegm1 = -(float)(dstsegm - 1);
-    float thr = kTiny;
-    if (dstsegm == 6) {
-        // the default DSTSEGM with its constant in the instructions (0.8 % faster)
-        for (int j = len2 >> 2; 0 <= j; j -= 2)
-            ddms_diagonal<true>(q, d + j, T, min(len1, len2 - j), 0, j, -5.0f, ms, mb, me, thr);
-        for (int i = len1 >> 2; 0 < i; i -= 2)
-            ddms_diagonal<true>(q + i, d, T, min(len2, len1 - i), i, 0, -5.0f, ms, mb, me, thr);
-    } else if (dstsegm >= 5) {
-        for (int j = len2 >> 2; 0 <= j; j -= 2)
-            ddms_diagonal<true>(q, d + j, T, min(len1, len2 - j), 0, j, nsegm1, ms, mb, me, thr);
-        for (int i = len1 >> 2; 0 < i; i -= 2)
-            ddms_diagonal<true>(q + i, d, T, min(len2, len1 - i), i, 0, nsegm1, ms, mb, me, thr);
-    } else {
-        for (int j = len2 >> 2; 0 <= j; j -= 2)
-            ddms_diagonal<false>(q, d + j, T, min(len1, len2 - j), 0, j, nsegm1, ms, mb, me, thr);
-        for (int i = len1 >> 2; 0 < i; i -= 2)
-            ddms_diagonal<false>(q + i, d, T, min(len2, len1 - i), i, 0, nsegm1, ms, mb, me, thr);
+    const LenMask lm = len_mask<kSeg>(dst);
+    DdmsReg r;
+    const uint8_t* db = reinterpret_cast<const uint8_t*>(d);
+    {
+        const int par = ((len2 >> 2) & 1) * kHalfWords;
+        for (int j = len2 >> 2; 0 <= j; j -= 2) {
+            const int n0 = j >> 1;
+            ddms_diagonal<true, kSeg>(q + 4, q[3], d + par + 1 + (n0 >> 2), 0x3210u + 0x1111u * (uint32_t)(n0 & 3),
+                                      db[4 * par + 3 + n0], T, min(len1, len2 - j), (uint32_t)j,
+                                      dst, lm, ks, r);
+        }
+    }
+    for (int i = len1 >> 2; 0 < i; i -= 2) {
+        const int n0 = i >> 1;
+        const uint32_t* ql = q + kQUp + ((n0 & 1) ? kQLow + n0 : n0 + 1);   // element n0
+        ddms_diagonal<false, kSeg>(ql + 1, ql[0], d + 1, 0u, db[3], T, min(len2, len1 - i),
+                                   (uint32_t)i << 16, dst, lm, ks, r);
     }
     float sum = 0.0f;
-    sum = sum + ms[0];
-    sum = sum + ms[1];
-    sum = sum + ms[2];
+    sum = sum + r.m0;
+    sum = sum + r.m1;
+    sum = sum + (r.m2 > kTiny ? r.m2 : 0.0f);
     return sum * 128.0f;
 }
 
@@ -267,20 +325,21 @@ __device__ __forceinline__ float cvs_cell(const ScoreArgs& a, const float* __res
 }
 
 // kRows query positions per block (8, 16 or 32; each warp takes every
-// kWarps-th of them), chosen by the tuner. kStacked: the rows belong to
+// kWarps-th of them), chosen by the tuner. kDdms: with the distance term (a
+// search without it needs neither its lists nor its registers). kStacked: the rows belong to
 // several queries (cbp_process_batch), each with its own background; a
 // separate instantiation, so that the single-query kernel is unchanged.
-template <int kRows, bool kStacked>
-__global__ void __launch_bounds__(kThreads, 10)
+template <int kRows, bool kStacked, bool kDdms>
+__global__ void __launch_bounds__(kThreads, 8)
 score_matrix_kernel(const ScoreArgs a)
 {
     __shared__ float s_dms[kDstCard * kDstCard];
     __shared__ float s_sst[kSSCard * kSSCard];
     // the distance lists: first packed at kDbCopy bytes as the bulk copies
-    // leave them, then at the odd stride kDbStride with the codes times 4
-    __shared__ __align__(16) uint8_t s_dbe[kCols * kDbCopy];
+    // leave them, then split by parity at the odd stride of kDbWords words
+    __shared__ __align__(16) uint32_t s_dbe[kCols * kDbWords];
     __shared__ __align__(8) unsigned long long s_bar;
-    __shared__ __align__(16) uint16_t s_qe[kRows * kElems];
+    __shared__ __align__(16) uint32_t s_qe[kRows * kQWords];
     __shared__ float s_dtf[kNAA][kCols];
     __shared__ float s_dbg[kNAA][kCols];
     __shared__ float s_dss[kNSS][kCols];
@@ -297,6 +356,8 @@ score_matrix_kernel(const ScoreArgs a)
     float (*s_qcvpn)[kRows] =
         reinterpret_cast<float (*)[kRows]>(s_cvsdyn + (kNCV + 2) * kCols + kRows * (kNCV + 1));
     __shared__ int s_col[kCols];
+    __shared__ __align__(16) uint32_t s_ks[4];
+    if (threadIdx.x < 4) s_ks[threadIdx.x] = 4u << (8 * threadIdx.x);
 
     const int tid = threadIdx.x;
     const int lane = tid & 31;
@@ -309,7 +370,7 @@ score_matrix_kernel(const ScoreArgs a)
         const int slot = colb + tid;
         s_col[tid] = slot < a.ncols ? (a.colorder ? a.colorder[slot] : slot) : -1;
     }
-    const bool ddms = a.ddmswgt > 0.0f;
+    constexpr bool ddms = kDdms;
     for (int i = tid; ddms && i < kDstCard * kDstCard; i += kThreads) s_dms[i] = a.dmstab[i] * 0x1p-7f;
     for (int i = tid; i < kSSCard * kSSCard; i += kThreads) s_sst[i] = a.sstab[i];
     if (ddms && tid == 0) {
@@ -327,7 +388,7 @@ score_matrix_kernel(const ScoreArgs a)
         const unsigned ncopy = __popc(__ballot_sync(0xffffffffu, cc >= 0));
         if (lane == 0) mbar_expect_tx(&s_bar, ncopy * (unsigned)kDbCopy);
         __syncwarp();
-        if (cc >= 0) bulk_load(s_dbe + lane * kDbCopy, a.db.dst + (a.col0 + cc) * kDstStride, kDbCopy, &s_bar);
+        if (cc >= 0) bulk_load(reinterpret_cast<char*>(s_dbe) + lane * kDbCopy, a.db.dst + (a.col0 + cc) * kDstStride, kDbCopy, &s_bar);
     }
 
     // database columns of this block: lane l takes slab column s_col[l]
@@ -380,17 +441,23 @@ score_matrix_kernel(const ScoreArgs a)
         }
     }
     if (tid < kRows) s_qlen[tid] = (rowb + tid < a.Lq) ? a.q.dstlen[rowb + tid] : 0;
-    // query lists: each code times 88, the byte offset of its table row
-    for (int idx = tid; ddms && idx < kRows * (kElems / 4); idx += kThreads) {
-        const int r = idx / (kElems / 4), w = idx - r * (kElems / 4);
+    // query lists as the diagonals read them: each code times 88, the byte
+    // offset of its table row
+    for (int idx = tid; ddms && idx < kRows * kQWords; idx += kThreads) {
+        const int r = idx / kQWords, w = idx - r * kQWords;
         const int row = rowb + r;
-        uint32_t v = 0x15151515u;
-        if (row < a.Lq) v = *reinterpret_cast<const uint32_t*>(a.q.dst + (long long)row * kDstStride + 4 * w);
-        uint16_t* o = s_qe + r * kElems + 4 * w;
-        o[0] = (uint16_t)((v & 0xffu) * (kDstCard * 4));
-        o[1] = (uint16_t)(((v >> 8) & 0xffu) * (kDstCard * 4));
-        o[2] = (uint16_t)(((v >> 16) & 0xffu) * (kDstCard * 4));
-        o[3] = (uint16_t)((v >> 24) * (kDstCard * 4));
+        uint32_t v = kDstNoData;
+        if (row < a.Lq) {
+            int e;
+            if (w < kQUp) {
+                e = 2 * (w - 3);
+            } else {
+                const int par = (a.q.dstlen[row] >> 2) & 1;
+                e = w < kQUp + kQLow ? 2 * (w - kQUp - 1) + par : 2 * (w - kQUp - kQLow) + par;
+            }
+            if (e >= 0 && e < kDstStride) v = a.q.dst[(long long)row * kDstStride + e];
+        }
+        s_qe[idx] = v * (kDstCard * 4);
     }
     if (ddms) {
         // the lists' copies: a wait that gives up flags the launch, waits
@@ -402,39 +469,46 @@ score_matrix_kernel(const ScoreArgs a)
             (void)mbar_wait_for(&s_bar, 0, kListWaitNs);
             return;
         }
-        // to the odd stride, each code times 4 (a byte offset in a row of
-        // the pair-score table; codes <= 21, so the shift never carries
-        // across bytes); a slot without a column reads as no data
+        // split by parity; a slot without a column and bytes past the
+        // list read as no data
         constexpr int kPer = (kCols * kDbWords + kThreads - 1) / kThreads;
-        const uint32_t* src = reinterpret_cast<const uint32_t*>(s_dbe);
+        const uint8_t* src = reinterpret_cast<const uint8_t*>(s_dbe);
         uint32_t w[kPer];
 #pragma unroll
         for (int k = 0; k < kPer; k++) {
             const int idx = tid + k * kThreads;
             const int c = idx / kDbWords, wd = idx - c * kDbWords;
-            w[k] = 0x15151515u;   // kDstNoData in every byte
-            if (idx < kCols * kDbWords && s_col[c] >= 0) w[k] = src[c * (kDbCopy / 4) + wd];
+            const int par = wd >= kHalfWords ? 1 : 0;
+            w[k] = 0;
+            for (int y = 0; y < 4; y++) {
+                const int e = 2 * (4 * (wd - par * kHalfWords) + y - 3) + par;
+                uint32_t v = kDstNoData;
+                if (idx < kCols * kDbWords && s_col[c] >= 0 && e >= 0 && e < kDbCopy) v = src[c * kDbCopy + e];
+                w[k] |= v << (8 * y);
+            }
         }
         __syncthreads();
-        uint32_t* dstw = reinterpret_cast<uint32_t*>(s_dbe);
 #pragma unroll
         for (int k = 0; k < kPer; k++) {
             const int idx = tid + k * kThreads;
-            if (idx < kCols * kDbWords) dstw[idx] = w[k] << 2;
+            if (idx < kCols * kDbWords) s_dbe[idx] = w[k];
         }
     }
     __syncthreads();
 
-    if (!cvalid) return;  // no block-wide synchronisation below
-
+    // no block-wide synchronisation below; a lane without a column stays
+    // with its warp (the DDMS runs by warps) and writes nothing
+    const uint4 ks = *reinterpret_cast<const uint4*>(s_ks);
     const int dlen = s_dlen[lane];
-    const uint8_t* de = s_dbe + lane * kDbStride;
+    const uint32_t* de = s_dbe + lane * kDbWords;
     const float dss0 = s_dss[0][lane], dss1 = s_dss[1][lane], dss2 = s_dss[2][lane];
 
     for (int r = warp; r < kRows; r += kWarps) {
         const int row = rowb + r;
         if (row >= a.Lq) break;
 
+        float s = 0.0f, mod = 0.0f;
+        if (cvalid) {
         // profile-profile term (CuBatchScoreMatrix_Init.cu:159-186)
         float acc = 0.0f;
         if (a.dots_in_scores) {
@@ -455,8 +529,7 @@ score_matrix_kernel(const ScoreArgs a)
                 acc = acc + __fdiv_rn(num, den);
             }
         }
-        float s = cb_logf(acc) - a.initshift;
-        float mod = 0.0f;
+        s = cb_logf(acc) - a.initshift;
         const float cvs = (a.cvswgt > 0.0f)
                               ? cvs_cell(a, s_qcv[r], s_qcvpn[0][r], s_qcvpn[1][r], s_dcv, lane,
                                          s_dcvpn[0][lane], s_dcvpn[1][lane])
@@ -501,15 +574,21 @@ score_matrix_kernel(const ScoreArgs a)
             s = s + cvs * a.cvswgt;
             mod = mod + (cvs - 0.5f) * a.cvswgt;
         }
+        }
 
         // DDMS term (CuBatchScoreMatrix_ddms2s_h2.cu:158-186)
-        if (a.ddmswgt > 0.0f) {
+        if constexpr (kDdms) {
             const int qlen = s_qlen[r];
-            if (qlen >= a.dstsegm && dlen >= a.dstsegm) {
-                const float sum = ddms_cell(s_qe + r * kElems, qlen, de, dlen,
-                                            reinterpret_cast<const char*>(s_dms), a.dstsegm);
+            const bool on = dlen >= a.dstsegm;
+            if (qlen >= a.dstsegm && __any_sync(kFull, on)) {
+                const char* T = reinterpret_cast<const char*>(s_dms);
+                const uint32_t* qe = s_qe + r * kQWords;
+                const int len2 = on ? dlen : 0;
+                const float sum = a.dstsegm == 6 ? ddms_cell<6>(qe, qlen, de, len2, T, a.dstsegm, ks)
+                                  : a.dstsegm >= 5 ? ddms_cell<5>(qe, qlen, de, len2, T, a.dstsegm, ks)
+                                                   : ddms_cell<1>(qe, qlen, de, len2, T, a.dstsegm, ks);
                 const float dm = __fmaf_rn(0.053f * 16.0f, sum, -1.235f) * a.ddmswgt;
-                if (dm != 0.0f) {
+                if (on && dm != 0.0f) {
                     // the modular score drops 0.2*DDMSWGT, in the contracted
                     // form of CuBatchScoreMatrix_ddms2s_h2.cu:171
                     s = s + dm;
@@ -517,9 +596,11 @@ score_matrix_kernel(const ScoreArgs a)
                 }
             }
         }
-        const long long o = (long long)row * a.ld + col;
-        a.scores[o] = s;
-        a.modscores[o] = mod;
+        if (cvalid) {
+            const long long o = (long long)row * a.ld + col;
+            a.scores[o] = s;
+            a.modscores[o] = mod;
+        }
     }
 }
 
@@ -570,15 +651,23 @@ void launch_column_order(const uint8_t* dstlen, long long col0, int ncols, long 
     CBP_CHECK_LAUNCH();
 }
 
-template <int kRows>
+template <int kRows, bool kStacked>
 void launch_score_rows(const ScoreArgs& a, cudaStream_t stream)
 {
     dim3 grid((unsigned)ceil_div(a.ncols, kCols), (unsigned)ceil_div(a.Lq, kRows));
     const size_t cvs_smem =
         a.cvswgt > 0.0f ? sizeof(float) * ((kNCV + 2) * kCols + kRows * (kNCV + 1) + 2 * kRows) : 0;
-    if (a.q.P > 1) score_matrix_kernel<kRows, true><<<grid, kThreads, cvs_smem, stream>>>(a);
-    else score_matrix_kernel<kRows, false><<<grid, kThreads, cvs_smem, stream>>>(a);
+    if (a.ddmswgt > 0.0f) score_matrix_kernel<kRows, kStacked, true><<<grid, kThreads, cvs_smem, stream>>>(a);
+    else score_matrix_kernel<kRows, kStacked, false><<<grid, kThreads, cvs_smem, stream>>>(a);
     CBP_CHECK_LAUNCH();
+}
+
+template <int kRows>
+void launch_score_rows(const ScoreArgs& a, cudaStream_t stream)
+{
+    // stacked queries (cbp_process_batch) have a background per row
+    if (a.q.P > 1) launch_score_rows<kRows, true>(a, stream);
+    else launch_score_rows<kRows, false>(a, stream);
 }
 
 void launch_score_matrix(const ScoreArgs& a, cudaStream_t stream)
