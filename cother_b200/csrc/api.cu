@@ -136,7 +136,7 @@ struct DevBuf {
 
 // Device copy of a packed profile set.
 struct ProfilesStore {
-    DevBuf tf, ss, dst, dstlen, trn, bkg, eno, plen, pstart, pro, aa, sss, cv, cvprior, cvnorm2;
+    DevBuf tf, ss, dst, dstlen, trn, bkg, eno, plen, pstart, order, pro, aa, sss, cv, cvprior, cvnorm2;
     ProfilesDev view;
     std::vector<int> h_plen;
     std::vector<long long> h_pstart;
@@ -151,13 +151,13 @@ struct ProfilesStore {
     ~ProfilesStore() { release(); }
     size_t bytes() const {
         size_t n = 0;
-        for (const DevBuf* b : {&tf, &ss, &dst, &dstlen, &trn, &bkg, &eno, &plen, &pstart, &pro, &aa,
+        for (const DevBuf* b : {&tf, &ss, &dst, &dstlen, &trn, &bkg, &eno, &plen, &pstart, &order, &pro, &aa,
                                 &sss, &cv, &cvprior, &cvnorm2})
             n += b->bytes;
         return n;
     }
     void release() {
-        for (DevBuf* b : {&tf, &ss, &dst, &dstlen, &trn, &bkg, &eno, &plen, &pstart, &pro, &aa, &sss,
+        for (DevBuf* b : {&tf, &ss, &dst, &dstlen, &trn, &bkg, &eno, &plen, &pstart, &order, &pro, &aa, &sss,
                           &cv, &cvprior, &cvnorm2})
             b->release();
         view = ProfilesDev();
@@ -410,6 +410,16 @@ void upload_profiles(ProfilesStore& st, char* const* beg, char* const* end, cuda
     for (size_t p = 0; p < P; p++)
         std::fill(pro.begin() + st.h_pstart[p], pro.begin() + st.h_pstart[p] + lens[p], (int)p);
 
+    // profiles by descending length (a counting sort; equal lengths in order)
+    std::vector<int> order(P);
+    {
+        std::vector<int> first(*std::max_element(lens, lens + P) + 2, 0);
+        const int top = (int)first.size() - 2;
+        for (size_t p = 0; p < P; p++) first[top - lens[p] + 1]++;
+        for (size_t k = 1; k < first.size(); k++) first[k] += first[k - 1];
+        for (size_t p = 0; p < P; p++) order[first[top - lens[p]]++] = (int)p;
+    }
+
     auto up = [&](DevBuf& b, const void* src, size_t bytes) {
         b.reserve(std::max<size_t>(bytes, 16));
         CBP_CUDA(cudaMemcpyAsync(b.p, src, bytes, cudaMemcpyHostToDevice, stream));
@@ -427,6 +437,7 @@ void upload_profiles(ProfilesStore& st, char* const* beg, char* const* end, cuda
     up(st.eno, beg[fENO], P * sizeof(float));
     up(st.plen, lens, P * sizeof(int));
     up(st.pstart, st.h_pstart.data(), P * sizeof(long long));
+    up(st.order, order.data(), P * sizeof(int));
     up(st.pro, pro.data(), N * sizeof(int));
     up(st.aa, beg[fAA], N);
     up(st.sss, beg[fSSstate], N);
@@ -445,6 +456,7 @@ void upload_profiles(ProfilesStore& st, char* const* beg, char* const* end, cuda
     v.dst = st.dst.as<uint8_t>(); v.dstlen = st.dstlen.as<uint8_t>();
     v.trn = st.trn.as<float>(); v.bkg = st.bkg.as<float>(); v.eno = st.eno.as<float>();
     v.plen = st.plen.as<int>(); v.pstart = st.pstart.as<long long>();
+    v.order = st.order.as<int>();
     v.pro = st.pro.as<int>(); v.aa = st.aa.as<int8_t>(); v.sss = st.sss.as<int8_t>();
     v.cv = with_cv ? st.cv.as<float>() : nullptr;
     v.cvprior = with_cv ? st.cvprior.as<float>() : nullptr;
@@ -847,6 +859,8 @@ void process_queries(cbp_context* c, size_t nq, const size_t* qlens, char* const
             d[k].col0 = s.col0;
             d[k].p0 = s.p0;
             d[k].nprof = s.p1 - s.p0;
+            // one slab of the whole chunk takes its profiles longest first
+            d[k].order = d[k].nprof == c->db->view.P ? c->db->view.order : nullptr;
             d[k].btck = c->btck.as<uint8_t>() + (long long)r.row0 * a.ld;
             d[k].bandbuf = c->bandbuf.as<float>();
             d[k].maxsc = c->dpmax.as<float>() + k * maxprof;

@@ -7,12 +7,14 @@
 // FinalizeDPPro (src/libmycu/cudp/CuBatchDP_final.cu:61-292) with a device
 // spin-lock + atomicAdd pass list.
 //
-// Here one warp owns one database profile for the whole DP: it sweeps bands
-// of 64 query rows, two per lane, along anti-diagonals (lane t is at column
-// s-t at step s). "Up" and "diagonal" states arrive from lane t-1 by
-// shuffle; lane 0 reads the bottom row of the previous band from a
-// per-profile global strip that lane 31 writes. One launch covers every
-// profile of a slab (no per-diagonal launches, no grid-wide syncs).
+// Here a warp sweeps bands of 64 query rows of one profile, two per lane,
+// along anti-diagonals (lane t is at column s-t at step s). "Up" and
+// "diagonal" states arrive from lane t-1 by shuffle; lane 0 reads the bottom
+// row of the previous band from a per-profile global strip that lane 31
+// writes. With many profiles one warp owns a profile; with few, the warps of a
+// block share one, each sweeping every W-th band behind the band above
+// (dp1_profile_warps). One launch covers every profile of a slab (no
+// per-diagonal launches, no grid-wide syncs).
 #include <cstdint>
 #include <type_traits>
 
@@ -37,8 +39,7 @@ __device__ __forceinline__ int corner_edge(int Lq, int Ld)
     return e > 60 ? 60 : e;
 }
 
-// The band layout. One warp owns one profile and sweeps bands of 64 query
-// rows, two per lane: lane t holds rows r0+2t (row "A") and r0+2t+1 (row
+// The band layout. A warp sweeps bands of 64 query rows, two per lane: lane t holds rows r0+2t (row "A") and r0+2t+1 (row
 // "B") and is at column s-t at step s. Row A takes its "up" states from
 // lane t-1's row B by shuffle, row B from the lane's own row A; so one
 // shuffle set, one read of the column's transitions and one ring index
@@ -167,19 +168,44 @@ __device__ __forceinline__ Q7 query_trn(const float* __restrict__ qtrn, long lon
     return q;
 }
 
-// kWarps warps (profiles) per block, each with its own DpStage in dynamic
-// shared memory. kBulk: score rows by bulk copies (the slab width is a
-// multiple of 4 floats and the buffers are aligned); otherwise by 4-byte
-// cp.async with the ring unshifted.
-template <int kWarps, bool kBulk, bool kCodes>
+// What the warps of one profile share (kShared): per warp the pieces of the
+// strip it has written, over all its bands, and its maximum; failed: a wait
+// gave up, the others stop.
+template <int kWarps>
+struct DpShare {
+    volatile int pieces[kWarps];
+    volatile int failed;
+    float best[kWarps];
+    int row[kWarps], col[kWarps];
+};
+
+// kWarps warps per block, each with its own DpStage in dynamic shared memory.
+// kShared: the block's warps sweep ONE profile, warp w its bands w, w +
+// kWarps, ..., each behind the band above; otherwise a profile each. The one
+// strip serves all bands: a band reads a piece of it before it writes it, and
+// the bands below wait for that write. Only consumers wait, so the waits form
+// a chain that ends at the first band, and each gives up after a second. kBulk:
+// score rows by bulk copies (the slab width is a multiple of 4 floats and the
+// buffers are aligned); otherwise by 4-byte cp.async with the ring unshifted.
+template <int kWarps, bool kShared, bool kBulk, bool kCodes>
 __global__ void __launch_bounds__(32 * kWarps)
 dp1_kernel(const Dp1Args a)
 {
     extern __shared__ __align__(128) unsigned char s_dyn[];
+    __shared__ DpShare<kShared ? kWarps : 1> sh;
     const int lane = threadIdx.x & 31;
-    const int pl = blockIdx.x * kWarps + (threadIdx.x >> 5);
-    if (pl >= a.nprof) return;  // whole warp
-    DpStage<kCodes>& st = reinterpret_cast<DpStage<kCodes>*>(s_dyn)[threadIdx.x >> 5];
+    const int warp = threadIdx.x >> 5;
+    const int slot = kShared ? blockIdx.x : blockIdx.x * kWarps + warp;
+    if (slot >= a.nprof) return;  // whole warp (kShared: whole block)
+    const int pl = a.order ? a.order[slot] : slot;
+    DpStage<kCodes>& st = reinterpret_cast<DpStage<kCodes>*>(s_dyn)[warp];
+    if (kShared) {
+        if (lane == 0) {
+            sh.pieces[kShared ? warp : 0] = 0;
+            if (warp == 0) sh.failed = 0;
+        }
+        __syncthreads();
+    }
     const int p = a.p0 + pl;
     const int Ld = a.db.plen[p];
     const long long colb = a.db.pstart[p] - a.col0;
@@ -187,7 +213,7 @@ dp1_kernel(const Dp1Args a)
         // a profile outside the slab's columns (or too long for the 16-bit
         // cell coordinates) is skipped: nothing of it is read or written,
         // and its maximum is flagged as NaN with coordinates 0xffffffff
-        if (lane == 0) {
+        if (lane == 0 && (!kShared || warp == 0)) {
             a.maxsc[pl] = Ld == 0 ? 0.0f : __int_as_float(0x7fc00000);
             a.maxcoords[pl] = Ld == 0 ? 0u : 0xffffffffu;
         }
@@ -228,7 +254,8 @@ dp1_kernel(const Dp1Args a)
         best = 0.0f;
         bestr = 0;
         bestc = 0;
-        for (int r0 = 0; r0 < Lq && ok; r0 += kBand) {
+        int nbands = 0;   // bands this warp has swept
+        for (int r0 = kShared ? kBand * warp : 0; r0 < Lq && ok; r0 += kShared ? kBand * kWarps : kBand) {
             const int rA = r0 + 2 * lane, rB = rA + 1;
             const bool vA = rA < Lq, vB = rB < Lq;
             const Q7 qa = query_trn(a.qtrn, QT, rA, Lq);
@@ -265,6 +292,24 @@ dp1_kernel(const Dp1Args a)
             float bstA = 0.0f, bstB = 0.0f;
             int bcA = 0, bcB = 0;
 
+            // kShared: until the warp of the band above has written piece h of
+            // the strip; false when it gave up or did not within a second
+            const int npieces = h_last + 1;
+            auto strip_ready = [&](int h) {
+                if (!kShared || top) return true;
+                const int w = warp == 0 ? kWarps - 1 : warp - 1;
+                const int need = (warp == 0 ? nbands - 1 : nbands) * npieces + h + 1;
+                unsigned long long t0 = 0;
+                bool got = true;
+                while (sh.pieces[kShared ? w : 0] < need) {
+                    const unsigned long long now = global_ns();
+                    if (t0 == 0) t0 = now;
+                    if (sh.failed || now - t0 > kWaitNs) { got = false; break; }
+                }
+                got = __all_sync(kFull, got);
+                __threadfence_block();   // the strip is read after its count
+                return got;
+            };
             // fetch piece h of this band into ring slot h mod 4
             auto issue = [&](int h) {
                 const int slot = h & (kSlots - 1);
@@ -376,6 +421,11 @@ dp1_kernel(const Dp1Args a)
                         strip[3 * ld + c] = v.w; strip[4 * ld + c] = st.sob[kPiece * slot + lane];
                     }
                 }
+                if (kShared && has_next) {
+                    __threadfence_block();
+                    __syncwarp();
+                    if (lane == 0) sh.pieces[kShared ? warp : 0] = nbands * npieces + h + 1;
+                }
             };
 
             // one step: cells (rA, c) and (rB, c) of the lane, c = s - lane.
@@ -449,6 +499,7 @@ dp1_kernel(const Dp1Args a)
             };
 
             __syncwarp();   // the previous band's tiles are no longer read
+            if (!strip_ready(0)) { ok = false; break; }   // no copy is in flight
             issue(0);
             int hflushed = 0;   // pieces 0 .. hflushed-1 are written back
             // steps with every lane inside the profile and on a row (the
@@ -463,7 +514,17 @@ dp1_kernel(const Dp1Args a)
                 if (H >= 3 && H - 3 <= h_last) { flush(H - 3); hflushed = H - 2; }
                 if (H <= h_last) {
                     const bool more = H + 1 <= h_last;
-                    if (more) issue(H + 1);
+                    if (more) {
+                        if (!strip_ready(H + 1)) {
+                            // piece H's copies end (or their wait gives up) first
+                            cp_async_commit();
+                            (void)await(H, false);
+                            cp_async_wait0();
+                            ok = false;
+                            break;
+                        }
+                        issue(H + 1);
+                    }
                     else cp_async_commit();   // an empty group keeps the wait accounting
                     if (!await(H, more)) { ok = false; break; }
                 }
@@ -492,7 +553,9 @@ dp1_kernel(const Dp1Args a)
             } else {
                 best = fmaxf(best, fmaxf(bstA, bstB));
             }
+            nbands++;
         }
+        if (kShared && !ok && lane == 0) sh.failed = 1;
     };
 
     // The codes are read only by the backtrace of a profile whose maximum
@@ -503,6 +566,13 @@ dp1_kernel(const Dp1Args a)
     if (!kCodes) {
         sweep(kFalse());
         for (int o = 16; o >= 1; o >>= 1) best = fmaxf(best, __shfl_xor_sync(kFull, best, o));
+        if (kShared) {
+            if (lane == 0) sh.best[kShared ? warp : 0] = best;
+            __syncthreads();
+            if (warp != 0) return;
+            for (int w = 1; w < kWarps; w++) best = fmaxf(best, sh.best[kShared ? w : 0]);
+            ok = !sh.failed;
+        }
         if (lane == 0) {
             // a staging wait that gave up flags the profile and the launch
             a.maxsc[pl] = ok ? best : __int_as_float(0x7fc00000);
@@ -512,8 +582,9 @@ dp1_kernel(const Dp1Args a)
         return;
     }
     if (a.code_thld != -INFINITY && !(a.maxsc[pl] > a.code_thld)) return;   // not a candidate
+    if (kShared) __syncthreads();   // every warp has read the maximum that warp 0 replaces
     sweep(kTrue());
-    if (!ok) {
+    if (!kShared && !ok) {
         if (lane == 0) {
             a.maxsc[pl] = __int_as_float(0x7fc00000);
             a.maxcoords[pl] = 0xffffffffu;
@@ -528,6 +599,30 @@ dp1_kernel(const Dp1Args a)
         const int oc = __shfl_xor_sync(kFull, bestc, o);
         if (best < ob || (best == ob && (orr < bestr || (orr == bestr && oc < bestc)))) {
             best = ob; bestr = orr; bestc = oc;
+        }
+    }
+    if (kShared) {
+        if (lane == 0) {
+            sh.best[kShared ? warp : 0] = best;
+            sh.row[kShared ? warp : 0] = bestr;
+            sh.col[kShared ? warp : 0] = bestc;
+        }
+        __syncthreads();
+        if (warp != 0) return;
+        for (int w = 1; w < kWarps; w++) {
+            const float ob = sh.best[kShared ? w : 0];
+            const int orr = sh.row[kShared ? w : 0], oc = sh.col[kShared ? w : 0];
+            if (best < ob || (best == ob && (orr < bestr || (orr == bestr && oc < bestc)))) {
+                best = ob; bestr = orr; bestc = oc;
+            }
+        }
+        if (sh.failed) {
+            if (lane == 0) {
+                a.maxsc[pl] = __int_as_float(0x7fc00000);
+                a.maxcoords[pl] = 0xffffffffu;
+                if (a.err) atomicExch(a.err, 1);
+            }
+            return;
         }
     }
     if (lane == 0) {
@@ -661,33 +756,82 @@ pass_compact_kernel(const Dp1Args a, int* __restrict__ pass_idx, long long* __re
 
 }  // namespace
 
-template <int kW, bool kBulk, bool kCodes>
+template <int kW, bool kShared, bool kBulk, bool kCodes>
 void launch_dp1_variant(const Dp1Args& a, cudaStream_t stream)
 {
     const size_t smem = (size_t)kW * sizeof(DpStage<kCodes>);
-    dp1_kernel<kW, kBulk, kCodes><<<(unsigned)ceil_div(a.nprof, kW), 32 * kW, smem, stream>>>(a);
+    dp1_kernel<kW, kShared, kBulk, kCodes>
+        <<<(unsigned)(kShared ? a.nprof : ceil_div(a.nprof, kW)), 32 * kW, smem, stream>>>(a);
     CBP_CHECK_LAUNCH();
+}
+
+template <int kW, bool kShared, bool kBulk, bool kCodes>
+void set_dp1_attribute()
+{
+    CBP_CUDA(cudaFuncSetAttribute(dp1_kernel<kW, kShared, kBulk, kCodes>,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kW * sizeof(DpStage<kCodes>))));
+}
+
+template <bool kCodes>
+void set_dp1_attributes()
+{
+    // dynamic shared memory above 48 KB needs an opt-in
+    set_dp1_attribute<2, false, true, kCodes>();
+    set_dp1_attribute<2, false, false, kCodes>();
+    set_dp1_attribute<2, true, true, kCodes>();
+    set_dp1_attribute<4, true, true, kCodes>();
+    set_dp1_attribute<8, true, true, kCodes>();
 }
 
 void dp1_set_attributes()
 {
-    // dynamic shared memory above 48 KB (two warps per block) needs an opt-in
-    CBP_CUDA(cudaFuncSetAttribute(dp1_kernel<2, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)(2 * sizeof(DpStage<true>))));
-    CBP_CUDA(cudaFuncSetAttribute(dp1_kernel<2, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)(2 * sizeof(DpStage<true>))));
-    CBP_CUDA(cudaFuncSetAttribute(dp1_kernel<2, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)(2 * sizeof(DpStage<false>))));
-    CBP_CUDA(cudaFuncSetAttribute(dp1_kernel<2, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)(2 * sizeof(DpStage<false>))));
+    set_dp1_attributes<true>();
+    set_dp1_attributes<false>();
+}
+
+// The warps of a profile. A single warp takes about 400 cycles a step (the
+// chain shuffle - row A - row B, at one warp's issue rate), so a launch of few
+// profiles is as long as its longest one; W warps sweep W bands at once, each
+// four 16-column pieces behind the band above, for W stages of shared memory
+// and the wavefront's filling. The lines lie where the measured times cross
+// (maxima of every profile and codes of 1 %; Lq x profiles of the 220-median
+// length law: ms with 1 / 2 / 4 / 8 warps): 400 x 300: 2.58 / 1.67 / 0.96 /
+// 0.83; 400 x 600: 2.70 / 1.81 / 1.11 / 1.25; 400 x 3,000: 4.02 / 3.12 / 2.97 /
+// 4.23; 200 x 3,000: 2.28 / 1.67 / 1.82 / 2.84; 400 x 8,000: 7.21 / 6.22 / 6.89;
+// 400 x 12,000: 7.63 / 7.62 / 9.56; 1,500 x 60 of 500-1,500: 18.96 / 10.99 /
+// 5.66 / 3.53.
+int dp1_profile_warps(int nprof, int Lq)
+{
+    constexpr int kSMs = 148;
+    const int nb = (Lq + kBand - 1) / kBand;
+    if (nb >= 5 && nprof <= 3 * kSMs) return 8;
+    if (nb >= 3 && nprof <= 16 * kSMs) return 4;
+    if (nb >= 2 && nprof <= 64 * kSMs) return 2;
+    return 1;
 }
 
 template <bool kCodes>
 void launch_dp1_pass(const Dp1Args& a, bool bulk, cudaStream_t stream)
 {
+    // a codes launch behind one for the maxima sweeps the candidates alone,
+    // about 1 % of a large database: at most an eighth is allowed for
+    const int work = kCodes && a.code_thld != -INFINITY ? (a.nprof + 7) / 8 : a.nprof;
+    const int share = bulk ? dp1_profile_warps(work, a.Lq) : 1;
+    switch (share) {
+    case 8: launch_dp1_variant<8, true, true, kCodes>(a, stream); return;
+    case 4: launch_dp1_variant<4, true, true, kCodes>(a, stream); return;
+    case 2: launch_dp1_variant<2, true, true, kCodes>(a, stream); return;
+    default: break;
+    }
     switch (a.warps) {
-    case 1: bulk ? launch_dp1_variant<1, true, kCodes>(a, stream) : launch_dp1_variant<1, false, kCodes>(a, stream); break;
-    case 2: bulk ? launch_dp1_variant<2, true, kCodes>(a, stream) : launch_dp1_variant<2, false, kCodes>(a, stream); break;
+    case 1:
+        bulk ? launch_dp1_variant<1, false, true, kCodes>(a, stream)
+             : launch_dp1_variant<1, false, false, kCodes>(a, stream);
+        break;
+    case 2:
+        bulk ? launch_dp1_variant<2, false, true, kCodes>(a, stream)
+             : launch_dp1_variant<2, false, false, kCodes>(a, stream);
+        break;
     default: throw Error(CBP_ERR_ARG, "phase-1 DP warps per block must be 1 or 2");
     }
 }

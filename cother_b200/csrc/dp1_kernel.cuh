@@ -32,7 +32,10 @@ struct Dp1Args {
     float* maxsc = nullptr;          // [nprof]
     uint32_t* maxcoords = nullptr;   // [nprof]
     Dp1Rec* recs = nullptr;          // [nprof]
-    int warps = 2;                   // warps (profiles) per block of dp1_kernel: 1 or 2
+    int warps = 2;                   // warps per block where each sweeps a profile of its own: 1 or 2
+    // the order the launches take the slab's profiles in, [nprof] (longest
+    // first, so that no long one is left for the end); null: as they come
+    const int* order = nullptr;
     int* err = nullptr;              // set to 1 when a staging wait gave up (may be null)
     // backtrack codes are computed for the profiles whose maximum exceeds
     // code_thld (the finalization's threshold: it backtraces only those);
@@ -45,6 +48,9 @@ struct Dp1Args {
 // profile's maximum and a second one sweeps the candidates again with codes
 // (2), with code_thld = -inf the second alone, for all profiles (1).
 int launch_dp1(const Dp1Args& a, cudaStream_t stream);
+// Warps that sweep one profile together in a launch of nprof profiles (1, 2,
+// 4 or 8); with 1, Dp1Args::warps profiles share a block.
+int dp1_profile_warps(int nprof, int Lq);
 // Per device, before the first launch_dp1 with two warps per block (and
 // outside any stream capture): the shared-memory opt-in of the DP kernels.
 void dp1_set_attributes();

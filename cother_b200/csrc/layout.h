@@ -13,7 +13,8 @@
 //    position instead of the reference's 400 B of floats.
 //  * transitions          trn  [7][N+P]   float  (entry pstart[p]+p is the
 //    beginning vector of profile p, entry pstart[p]+p+1+k its position k)
-//  * per profile          bkg [20][P], eno [P], plen [P], pstart [P]
+//  * per profile          bkg [20][P], eno [P], plen [P], pstart [P], order
+//                         [P] (profile indices by descending length)
 //  * per position         pro [N] (profile index), aa [N], sss [N]
 #pragma once
 
@@ -47,6 +48,7 @@ struct ProfilesDev {
     const int* plen = nullptr;
     const long long* pstart = nullptr;
     const int* pro = nullptr;
+    const int* order = nullptr;      // [P] profiles by descending length
     const int8_t* aa = nullptr;
     const int8_t* sss = nullptr;
     // context vectors, when uploaded: [19][N] entries, [N] log priors, [N]
