@@ -48,12 +48,12 @@ __device__ __forceinline__ int corner_edge(int Lq, int Ld)
 // only set the column -1 states of each row and the diagonal of a band's
 // last row at column 0, which are reproduced per row (row mod 32).
 //
-// Steps. While every lane is inside the profile (steps 32 .. Ld-1 of a
-// band whose 64 rows all exist) a step runs without predicates: no column
-// or row checks and no column-0 case. The first and last 32 steps of a
-// band (the wavefront filling and draining) and a last band of fewer rows
-// use the checked step; a partial band ends when its last valid lane
-// leaves the profile.
+// Steps. While every lane that holds a row is inside the profile (steps 32
+// .. Ld-1 of a whole band) a step runs without predicates: no column or row
+// checks and no column-0 case. The first and last steps of a band (the
+// wavefront filling and draining) use the checked step; a last band of fewer
+// rows ends when its last valid lane leaves the profile (with the checked
+// step throughout, a query of 40 took 0.27 ms against 16 profiles).
 //
 // Staging. The band's columns are staged in pieces of 16 through a ring of
 // 64 columns in shared memory: piece h+1 is fetched while the warp sweeps
@@ -262,7 +262,6 @@ dp1_kernel(const Dp1Args a)
             const Q7 qb = query_trn(a.qtrn, QT, rB, Lq);
             const bool top = (r0 == 0);
             const bool has_next = r0 + kBand < Lq;
-            const bool full = r0 + kBand <= Lq;           // all 64 rows exist
             const int nlanes = min(32, (Lq - r0 + 1) >> 1);   // lanes holding a row
             const int nsteps = Ld + nlanes - 1;
             const bool lastB = (rB & 31) == 31;  // the last row of a 32-row band of the reference
@@ -502,9 +501,11 @@ dp1_kernel(const Dp1Args a)
             if (!strip_ready(0)) { ok = false; break; }   // no copy is in flight
             issue(0);
             int hflushed = 0;   // pieces 0 .. hflushed-1 are written back
-            // steps with every lane inside the profile and on a row (the
-            // unchecked steps): [32, Ld) on a full band
-            const int fast0 = full ? 32 : nsteps, fast1 = full ? Ld : nsteps;
+            // steps with every lane that holds a row inside the profile, past
+            // column 0 (the unchecked steps); lanes and rows past the last
+            // query row compute what nothing reads: states pass from a lane
+            // to the next one only
+            const int fast0 = nlanes, fast1 = Ld;
             for (int H = 0;; H++) {
                 const int sb = (H == 0) ? 0 : kPiece * H - off;   // lane 0 enters piece H
                 if (sb >= nsteps) break;
@@ -548,10 +549,11 @@ dp1_kernel(const Dp1Args a)
             for (int h = hflushed; h <= h_last; h++) flush(h);
             // the band's maxima into the lane's, in row-major order
             if (kSweepCodes) {
-                if (best < bstA) { best = bstA; bestr = rA; bestc = bcA; }
-                if (best < bstB) { best = bstB; bestr = rB; bestc = bcB; }
+                if (vA && best < bstA) { best = bstA; bestr = rA; bestc = bcA; }
+                if (vB && best < bstB) { best = bstB; bestr = rB; bestc = bcB; }
             } else {
-                best = fmaxf(best, fmaxf(bstA, bstB));
+                if (vA) best = fmaxf(best, bstA);
+                if (vB) best = fmaxf(best, bstB);
             }
             nbands++;
         }
