@@ -481,7 +481,7 @@ void check_ctx(cbp_context* c)
 size_t slab_bytes_per_position(const cbp_options& o, int Lq)
 {
     const size_t nb = (size_t)map_bands(Lq);
-    size_t b = (size_t)Lq * 9 + 172 + nb * (8 * 32 + 12) + 4 * kMapMaxWarps * kMapEdgeFields + 5 +
+    size_t b = (size_t)Lq * 9 + 172 + nb * (8 * 32 + 12) + 4 * kMapStrips * kMapEdgeFields + 5 +
                (size_t)Lq * 5;
     (void)o;   // the tensor-core form needs only the query's operand image (per query, not per position)
     return b;

@@ -329,21 +329,29 @@ __device__ __forceinline__ EdgeLink edge_link(const MapArgs& a, const Pair& q, i
 {
     EdgeLink e;
     const int Ld = q.Ld;
-    float* strips = a.strip + (long long)kMapMaxWarps * kMapEdgeFields * q.dst;
+    float* strips = a.strip + (long long)kMapStrips * kMapEdgeFields * q.dst;
     e.nce = (Ld + 31) >> 5;
     e.has_in = o > 0;
     e.islot = (o + W - 1) % W;
     e.ibase = o > 0 ? ((o - 1) / W) * e.nce : 0;
     e.obase = (o / W) * e.nce;
-    e.in = strips + (long long)e.islot * kMapEdgeFields * Ld;
-    e.out = strips + (long long)w * kMapEdgeFields * Ld;
+    // warps kMapStrips apart share a strip: a band writes a position after its
+    // read of that position, which follows the write of the band above, and so
+    // on up to the band that reads what is overwritten
+    e.in = strips + (long long)(e.islot % kMapStrips) * kMapEdgeFields * Ld;
+    e.out = strips + (long long)(w % kMapStrips) * kMapEdgeFields * Ld;
     return e;
 }
 
 // Edge chunk J (positions 32J..32J+31) is read during steps 32J..32J+31;
-// chunk J+1 is loaded into registers at step 32J. The writer publishes at
-// step 32J the J-1 chunks it has completed (position u is written at step
-// u+31) and all of them at the end of the band.
+// chunk J+1 is loaded into registers at step 32J + kEdgeAhead, a few steps
+// (several load latencies) before its use. The writer publishes at step 32J
+// the J-1 chunks it has completed (position u is written at step u+31) and all
+// of them at the end of the band. So a band runs 68 steps behind the one
+// above (96 when the next chunk was loaded at step 32J: 1,000 x 100 2.87 ms
+// against 2.49 ms).
+constexpr int kEdgeAhead = 28;
+
 template <int NF>
 __device__ __forceinline__ void edge_prologue(BlockShared& sh, WarpStage& st, const EdgeLink& e,
                                               int Ld, float (&er)[NF], int* err, int lane)
@@ -352,23 +360,15 @@ __device__ __forceinline__ void edge_prologue(BlockShared& sh, WarpStage& st, co
     wait_chunks(sh, e.islot, e.ibase + 1, err);
     load_edge<NF>(er, e.in, Ld, 0, lane);
     store_edge<NF>(st, er, 0, lane);
-    if (e.nce > 1) {
-        wait_chunks(sh, e.islot, e.ibase + 2, err);
-        load_edge<NF>(er, e.in, Ld, 1, lane);
-    }
 }
 
 template <int NF>
-__device__ __forceinline__ void edge_chunk_start(BlockShared& sh, WarpStage& st, const EdgeLink& e,
-                                                 int Ld, float (&er)[NF], int J, int* err, int lane)
+__device__ __forceinline__ void edge_load_next(BlockShared& sh, const EdgeLink& e, int Ld, float (&er)[NF], int J,
+                                               int* err, int lane)
 {
-    if (!e.has_in) return;
-    if (J < e.nce) store_edge<NF>(st, er, J, lane);
-    __syncwarp();
-    if (J + 1 < e.nce) {
-        wait_chunks(sh, e.islot, e.ibase + J + 2, err);
-        load_edge<NF>(er, e.in, Ld, J + 1, lane);
-    }
+    if (!e.has_in || J + 1 >= e.nce) return;
+    wait_chunks(sh, e.islot, e.ibase + J + 2, err);
+    load_edge<NF>(er, e.in, Ld, J + 1, lane);
 }
 
 // One diagonal row of a band into the per-lane ring, kRows - 1 steps ahead,
@@ -481,12 +481,15 @@ __device__ __forceinline__ float forward_pass(const MapArgs& a, const Pair& q, B
             if (J > 0) {
                 __syncwarp();
                 store_trn(st, tr, J + 1, lane);
-                edge_chunk_start<5>(sh, st, e, Ld, er, J, a.err, lane);
+                if (e.has_in && J < e.nce) store_edge<5>(st, er, J, lane);
                 __syncwarp();
                 load_trn(tr, dtr, NT, Ld, J + 2, false, lane);
                 if (lane == 31 && J >= 2) publish(sh, w, e.obase + J - 1);
             }
-            run_steps(s0, s1, J > 0 && s1 <= Ld, step);
+            const int sm = min(s0 + kEdgeAhead, s1);
+            run_steps(s0, sm, J > 0 && s1 <= Ld, step);
+            edge_load_next<5>(sh, e, Ld, er, J, a.err, lane);
+            run_steps(sm, s1, J > 0 && s1 <= Ld, step);
         }
         cp_wait<0>();
         if (lane == 31) publish(sh, w, e.obase + e.nce);
@@ -601,12 +604,15 @@ __device__ __forceinline__ void backward_pass(const MapArgs& a, const Pair& q, B
             if (J > 0) {
                 __syncwarp();
                 store_trn(st, tr, J + 1, lane);
-                edge_chunk_start<6>(sh, st, e, Ld, er, J, a.err, lane);
+                if (e.has_in && J < e.nce) store_edge<6>(st, er, J, lane);
                 __syncwarp();
                 load_trn(tr, dtr, NT, Ld, J + 2, true, lane);
                 if (lane == 0 && J >= 2) publish(sh, w, e.obase + J - 1);
             }
-            run_steps(s0, s1, J > 0 && s1 <= Ld, step);
+            const int sm = min(s0 + kEdgeAhead, s1);
+            run_steps(s0, sm, J > 0 && s1 <= Ld, step);
+            edge_load_next<6>(sh, e, Ld, er, J, a.err, lane);
+            run_steps(sm, s1, J > 0 && s1 <= Ld, step);
         }
         cp_wait<0>();
         if (lane == 0) publish(sh, w, e.obase + e.nce);
@@ -686,10 +692,14 @@ __device__ __forceinline__ Best map_pass(const MapArgs& a, const Pair& q, BlockS
             const int s0 = 32 * J, s1 = min(s0 + 32, nsteps);
             if (J > 0) {
                 __syncwarp();
-                edge_chunk_start<1>(sh, st, e, Ld, er, J, a.err, lane);
+                if (e.has_in && J < e.nce) store_edge<1>(st, er, J, lane);
+                __syncwarp();
                 if (lane == 31 && J >= 2) publish(sh, w, e.obase + J - 1);
             }
-            run_steps(s0, s1, J > 0 && s1 <= Ld, step);
+            const int sm = min(s0 + kEdgeAhead, s1);
+            run_steps(s0, sm, J > 0 && s1 <= Ld, step);
+            edge_load_next<1>(sh, e, Ld, er, J, a.err, lane);
+            run_steps(sm, s1, J > 0 && s1 <= Ld, step);
         }
         cp_wait<0>();
         if (lane == 31) publish(sh, w, e.obase + e.nce);
@@ -698,7 +708,7 @@ __device__ __forceinline__ Best map_pass(const MapArgs& a, const Pair& q, BlockS
     return best;
 }
 
-__global__ void __launch_bounds__(32 * kMapMaxWarps, 2)
+__global__ void __launch_bounds__(32 * kMapMaxWarps)
 map_kernel(const MapArgs a, int nb)
 {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -974,6 +984,16 @@ void launch_aln_final(const MapArgs& a, const uint8_t* btck1, const float* maxsc
     CBP_CHECK_LAUNCH();
 }
 
+// Warps of a pair. Few pairs leave SMs idle and take as long as their bands'
+// chain, of which 16 warps, four to a scheduler, overlap more: 1,500 x 60
+// 10.2 ms with 8 and 8.2 ms with 16, 400 x 500 2.45 and 2.19 ms. With a pair for
+// every SM, 8: two such blocks share an SM.
+static int map_pair_warps(int npass, int nb)
+{
+    const int most = npass <= 148 ? kMapMaxWarps : kMapMaxWarps / 2;
+    return nb < most ? nb : most;
+}
+
 void launch_map(const MapArgs& a, cudaStream_t stream)
 {
     if (a.npass <= 0) return;
@@ -984,7 +1004,7 @@ void launch_map(const MapArgs& a, cudaStream_t stream)
     const dim3 sgrid((unsigned)ceil_div(units, kScoreWarps), 16);
     map_scores_kernel<<<sgrid, 32 * kScoreWarps, 0, stream>>>(a, nb);
     CBP_CHECK_LAUNCH();
-    const int W = nb < kMapMaxWarps ? nb : kMapMaxWarps;
+    const int W = map_pair_warps(a.npass, nb);
     const size_t smem = kSharedHead + (size_t)W * sizeof(WarpStage) + (size_t)nb * sizeof(float);
     CBP_CUDA(cudaFuncSetAttribute(map_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     map_kernel<<<a.npass, 32 * W, smem, stream>>>(a, nb);

@@ -14,7 +14,8 @@ namespace cbp {
 // of an anti-diagonal sweep are one contiguous 128-byte row. A band has
 // `nd` = phase-2 positions + 31 diagonal rows; neighbouring pairs share
 // their first and last 31 rows, in disjoint lanes.
-constexpr int kMapMaxWarps = 8;     // warps (32-row bands in flight) per pair
+constexpr int kMapMaxWarps = 16;    // warps (32-row bands in flight) per pair
+constexpr int kMapStrips = 8;       // band-edge strips per pair
 constexpr int kMapEdgeFields = 6;   // floats per column of a band edge
 
 struct MapArgs {
@@ -41,7 +42,7 @@ struct MapArgs {
     float* fb = nullptr;                // [nb][nd][32] forward, then forward + backward, log MM
     unsigned* sg = nullptr;             // [nb][nd] bit t: raw score of row 32b+t > 0
     unsigned long long* bt = nullptr;   // [nb][nd] MAP backtrack codes: bit t | bit 32+t
-    float* strip = nullptr;             // [kMapMaxWarps][6][Ld] band edges per pair, at 48*pass_dst
+    float* strip = nullptr;             // [kMapStrips][6][Ld] band edges per pair, at 48*pass_dst
     int* err = nullptr;                 // set when a wait between warps gives up
     char* alns = nullptr;               // [5][alnstride] alignment rows
     long long alnstride = 0;
@@ -51,7 +52,7 @@ inline long long map_diag_rows(long long npos2) { return npos2 + 31; }
 inline long long map_bands(int Lq) { return (Lq + 31) / 32; }
 inline long long map_strip_floats(long long npos2)
 {
-    return (long long)kMapMaxWarps * kMapEdgeFields * npos2;
+    return (long long)kMapStrips * kMapEdgeFields * npos2;
 }
 
 // zeroes sg and bt, then realigns every pair of the pass list
