@@ -134,9 +134,29 @@ struct DevBuf {
     template <class T> T* as() const { return static_cast<T*>(p); }
 };
 
+// A page-locked host buffer that only grows: what a small upload or read-back
+// is staged in, so that it is one asynchronous copy.
+struct PinBuf {
+    void* p = nullptr;
+    size_t bytes = 0;
+    void reserve(size_t n) {
+        if (n <= bytes) return;
+        release();
+        CBP_CUDA(cudaHostAlloc(&p, n, cudaHostAllocDefault));
+        bytes = n;
+    }
+    void release() {
+        if (p) cudaFreeHost(p);
+        p = nullptr; bytes = 0;
+    }
+    template <class T> T* as() const { return static_cast<T*>(p); }
+};
+constexpr size_t kMaxStaged = 4u << 20;   // larger copies go straight to their places
+
 // Device copy of a packed profile set.
 struct ProfilesStore {
     DevBuf tf, ss, dst, dstlen, trn, bkg, eno, plen, pstart, order, pro, aa, sss, cv, cvprior, cvnorm2;
+    DevBuf blob;                     // a small set: all of the above in one buffer
     ProfilesDev view;
     std::vector<int> h_plen;
     std::vector<long long> h_pstart;
@@ -152,13 +172,13 @@ struct ProfilesStore {
     size_t bytes() const {
         size_t n = 0;
         for (const DevBuf* b : {&tf, &ss, &dst, &dstlen, &trn, &bkg, &eno, &plen, &pstart, &order, &pro, &aa,
-                                &sss, &cv, &cvprior, &cvnorm2})
+                                &sss, &cv, &cvprior, &cvnorm2, &blob})
             n += b->bytes;
         return n;
     }
     void release() {
         for (DevBuf* b : {&tf, &ss, &dst, &dstlen, &trn, &bkg, &eno, &plen, &pstart, &order, &pro, &aa, &sss,
-                          &cv, &cvprior, &cvnorm2})
+                          &cv, &cvprior, &cvnorm2, &blob})
             b->release();
         view = ProfilesDev();
         h_plen.clear();
@@ -277,7 +297,8 @@ struct cbp_context {
     cudaGraphExec_t phase1_exec = nullptr;
     uint64_t graph_launches = 0;
     // instrumentation
-    cudaEvent_t ev[8]{};
+    cudaEvent_t ev[10]{};
+    PinBuf qpin, cpin, rpin;        // staging of the queries, the pass counts, the results
     float stage_ms[6] = {0, 0, 0, 0, 0, 0};
     uint64_t launches = 0;
     uint64_t stage_launches[6] = {0, 0, 0, 0, 0, 0};
@@ -324,9 +345,11 @@ size_t field_bytes(char* const* beg, char* const* end, int f)
 
 // Repack 181 SoA host fields into the device layout (layout.h) and upload.
 // Upload a packed profile set. With `with_cv` the context-vector fields
-// (pmv2DCVentrs.., pmv2DCVprior, pmv2DCVnorm2) are uploaded too.
+// (pmv2DCVentrs.., pmv2DCVprior, pmv2DCVnorm2) are uploaded too. With `pin` a
+// small set (queries) is packed there and goes up in one asynchronous copy
+// (its 60-odd copies from pageable memory and their wait took about 0.2 ms).
 void upload_profiles(ProfilesStore& st, char* const* beg, char* const* end, cudaStream_t stream,
-                     bool with_cv)
+                     bool with_cv, PinBuf* pin = nullptr)
 {
     if (!beg || !end) throw Error(CBP_ERR_ARG, "null field tables");
     const size_t P = field_bytes(beg, end, fLen) / sizeof(int);
@@ -374,33 +397,43 @@ void upload_profiles(ProfilesStore& st, char* const* beg, char* const* end, cuda
     }
 
     // packed distance lists
-    std::vector<uint8_t> dst((size_t)N * kDstStride);
+    std::vector<uint8_t> dst((size_t)N * kDstStride, (uint8_t)kDstNoData);
     std::vector<uint8_t> dlen(N);
     const float* dd[100];
     for (int s = 0; s < 100; s++) dd[s] = reinterpret_cast<const float*>(beg[fDD + s]);
     std::string perr;
     std::mutex emu;
     parallel_for((long long)N, [&](long long a, long long b) {
-        for (long long n = a; n < b; n++) {
-            const int cnt = (int)dd[0][n];
-            uint8_t* o = dst.data() + (size_t)n * kDstStride;
-            if (cnt < 0 || cnt > kMaxDst) {
-                std::lock_guard<std::mutex> g(emu);
-                perr = "distance count out of range at position " + std::to_string(n);
-                return;
-            }
-            dlen[n] = (uint8_t)cnt;
-            int k = 0;
-            for (; k < cnt; k++) {
-                int v = (int)dd[k + 1][n];
-                if (v < 0) {
+        // by blocks of positions, one list element of all of them at a time:
+        // the fields are read in order
+        constexpr long long kBlock = 64;
+        for (long long n0 = a; n0 < b; n0 += kBlock) {
+            const int m = (int)std::min(kBlock, b - n0);
+            int most = 0;
+            for (int i = 0; i < m; i++) {
+                const int cnt = (int)dd[0][n0 + i];
+                if (cnt < 0 || cnt > kMaxDst) {
                     std::lock_guard<std::mutex> g(emu);
-                    perr = "negative distance at position " + std::to_string(n);
+                    perr = "distance count out of range at position " + std::to_string(n0 + i);
                     return;
                 }
-                o[k] = (uint8_t)(v == 255 ? kDstNoData : (v < 20 ? v : 20));
+                dlen[n0 + i] = (uint8_t)cnt;
+                most = std::max(most, cnt);
             }
-            for (; k < kDstStride; k++) o[k] = (uint8_t)kDstNoData;
+            uint8_t* o = dst.data() + (size_t)n0 * kDstStride;
+            for (int k = 0; k < most; k++) {
+                const float* src = dd[k + 1] + n0;
+                for (int i = 0; i < m; i++) {
+                    if (k >= dlen[n0 + i]) continue;
+                    const int v = (int)src[i];
+                    if (v < 0) {
+                        std::lock_guard<std::mutex> g(emu);
+                        perr = "negative distance at position " + std::to_string(n0 + i);
+                        return;
+                    }
+                    o[(size_t)i * kDstStride + k] = (uint8_t)(v == 255 ? kDstNoData : (v < 20 ? v : 20));
+                }
+            }
         }
     });
     if (!perr.empty()) throw Error(CBP_ERR_ARG, perr);
@@ -421,15 +454,17 @@ void upload_profiles(ProfilesStore& st, char* const* beg, char* const* end, cuda
         for (size_t p = 0; p < P; p++) order[first[top - lens[p]]++] = (int)p;
     }
 
-    auto up = [&](DevBuf& b, const void* src, size_t bytes) {
-        b.reserve(std::max<size_t>(bytes, 16));
-        CBP_CUDA(cudaMemcpyAsync(b.p, src, bytes, cudaMemcpyHostToDevice, stream));
+    struct Part {
+        DevBuf* buf;
+        size_t bytes;                                 // of the buffer
+        std::vector<std::pair<const void*, size_t>> pieces;   // one after another
+        size_t base;                                  // in the blob
     };
+    std::vector<Part> parts;
+    auto up = [&](DevBuf& b, const void* src, size_t bytes) { parts.push_back({&b, bytes, {{src, bytes}}, 0}); };
     auto up_rows = [&](DevBuf& b, int f0, int nrows, size_t row_elems, size_t esz) {
-        b.reserve(std::max<size_t>(nrows * row_elems * esz, 16));
-        for (int r = 0; r < nrows; r++)
-            CBP_CUDA(cudaMemcpyAsync(b.as<char>() + r * row_elems * esz, beg[f0 + r], row_elems * esz,
-                                     cudaMemcpyHostToDevice, stream));
+        parts.push_back({&b, nrows * row_elems * esz, {}, 0});
+        for (int r = 0; r < nrows; r++) parts.back().pieces.emplace_back(beg[f0 + r], row_elems * esz);
     };
     up_rows(st.tf, fTF, kNAA, N, sizeof(float));
     up_rows(st.ss, fSS, kNSS, N, sizeof(float));
@@ -449,19 +484,52 @@ void upload_profiles(ProfilesStore& st, char* const* beg, char* const* end, cuda
         up(st.cvprior, beg[fCV + kNCV], N * sizeof(float));
         up(st.cvnorm2, beg[fCV + kNCV + 1], N * sizeof(float));
     }
-    CBP_CUDA(cudaStreamSynchronize(stream));
+    size_t total = 0;
+    for (Part& t : parts) {
+        t.base = total;
+        total += (size_t)align_up((long long)std::max<size_t>(t.bytes, 16), 256);
+    }
+    const bool small = pin && total <= kMaxStaged;
+    if (small) {
+        pin->reserve(total);
+        st.blob.reserve(total);
+        for (const Part& t : parts) {
+            char* o = pin->as<char>() + t.base;
+            for (const auto& x : t.pieces) {
+                std::memcpy(o, x.first, x.second);
+                o += x.second;
+            }
+        }
+        CBP_CUDA(cudaMemcpyAsync(st.blob.p, pin->p, total, cudaMemcpyHostToDevice, stream));
+    } else {
+        for (const Part& t : parts) {
+            t.buf->reserve(std::max<size_t>(t.bytes, 16));
+            char* o = t.buf->as<char>();
+            for (const auto& x : t.pieces) {
+                CBP_CUDA(cudaMemcpyAsync(o, x.first, x.second, cudaMemcpyHostToDevice, stream));
+                o += x.second;
+            }
+        }
+        CBP_CUDA(cudaStreamSynchronize(stream));
+    }
+    auto at = [&](const DevBuf& b) -> void* {
+        if (!small) return b.p;
+        for (const Part& t : parts)
+            if (t.buf == &b) return st.blob.as<char>() + t.base;
+        return nullptr;
+    };
 
     ProfilesDev& v = st.view;
     v.N = (long long)N; v.P = (int)P;
-    v.tf = st.tf.as<float>(); v.ss = st.ss.as<float>();
-    v.dst = st.dst.as<uint8_t>(); v.dstlen = st.dstlen.as<uint8_t>();
-    v.trn = st.trn.as<float>(); v.bkg = st.bkg.as<float>(); v.eno = st.eno.as<float>();
-    v.plen = st.plen.as<int>(); v.pstart = st.pstart.as<long long>();
-    v.order = st.order.as<int>();
-    v.pro = st.pro.as<int>(); v.aa = st.aa.as<int8_t>(); v.sss = st.sss.as<int8_t>();
-    v.cv = with_cv ? st.cv.as<float>() : nullptr;
-    v.cvprior = with_cv ? st.cvprior.as<float>() : nullptr;
-    v.cvnorm2 = with_cv ? st.cvnorm2.as<float>() : nullptr;
+    v.tf = (const float*)at(st.tf); v.ss = (const float*)at(st.ss);
+    v.dst = (const uint8_t*)at(st.dst); v.dstlen = (const uint8_t*)at(st.dstlen);
+    v.trn = (const float*)at(st.trn); v.bkg = (const float*)at(st.bkg); v.eno = (const float*)at(st.eno);
+    v.plen = (const int*)at(st.plen); v.pstart = (const long long*)at(st.pstart);
+    v.order = (const int*)at(st.order);
+    v.pro = (const int*)at(st.pro); v.aa = (const int8_t*)at(st.aa); v.sss = (const int8_t*)at(st.sss);
+    v.cv = with_cv ? (const float*)at(st.cv) : nullptr;
+    v.cvprior = with_cv ? (const float*)at(st.cvprior) : nullptr;
+    v.cvnorm2 = with_cv ? (const float*)at(st.cvnorm2) : nullptr;
 }
 
 void check_ctx(cbp_context* c)
@@ -706,12 +774,12 @@ void process_queries(cbp_context* c, size_t nq, const size_t* qlens, char* const
                                        "(transferred by a context with CVSWGT > 0)");
     }
     if (nq == 1) {
-        upload_profiles(c->query, qbeg[0], qend[0], c->stream, c->opt.cvswgt > 0.0f);
+        upload_profiles(c->query, qbeg[0], qend[0], c->stream, c->opt.cvswgt > 0.0f, &c->qpin);
         if (c->query.view.P != 1) throw Error(CBP_ERR_ARG, "the query field tables must hold one profile");
     } else {
         StackedTables t;
         stack_tables(nq, qbeg, qend, t);
-        upload_profiles(c->query, t.beg, t.end, c->stream, c->opt.cvswgt > 0.0f);
+        upload_profiles(c->query, t.beg, t.end, c->stream, c->opt.cvswgt > 0.0f, &c->qpin);
     }
     const int Ltot = (int)c->query.view.N;
     std::vector<QueryResult> res(nq);
@@ -945,11 +1013,20 @@ void process_queries(cbp_context* c, size_t nq, const size_t* qlens, char* const
         c->stage_launches[0] += 2;
         c->stage_launches[1] += (uint64_t)dp_launches;
         c->stage_launches[2] += 2 * (uint64_t)nq;
-        std::vector<int> npass(nq, 0);
-        for (size_t k = 0; k < nq; k++)
-            CBP_CUDA(cudaMemcpyAsync(&npass[k], pass_cnt(k), sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-        CBP_CUDA(cudaMemcpyAsync(&c->h_dp1err, c->dp1err.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+        // the pass counts and phase-2 positions of all queries, and the flag of
+        // the launches' waits
+        c->cpin.reserve(nq * 16 + sizeof(int));
+        int* const flag = reinterpret_cast<int*>(c->cpin.as<char>() + nq * 16);
+        CBP_CUDA(cudaMemcpyAsync(c->cpin.p, c->passcnt.p, nq * 16, cudaMemcpyDeviceToHost, c->stream));
+        CBP_CUDA(cudaMemcpyAsync(flag, c->dp1err.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
         CBP_CUDA(cudaStreamSynchronize(c->stream));
+        c->h_dp1err = *flag;
+        std::vector<int> npass(nq, 0);
+        std::vector<long long> npos(nq, 0);
+        for (size_t k = 0; k < nq; k++) {
+            std::memcpy(&npass[k], c->cpin.as<char>() + 16 * k, sizeof(int));
+            std::memcpy(&npos[k], c->cpin.as<char>() + 16 * k + 8, sizeof(long long));
+        }
         if (c->h_dp1err == 2)
             throw Error(CBP_ERR_CUDA, "score matrix: a wait for the bulk-copied distance lists timed out");
         if (c->h_dp1err)
@@ -1021,10 +1098,7 @@ void process_queries(cbp_context* c, size_t nq, const size_t* qlens, char* const
 
             // phase-2 MAP realignment of the pairs within the E-value
             // threshold (in the phase-2 column space of this slab)
-            long long npos2 = 0;
-            CBP_CUDA(cudaMemcpyAsync(&npos2, pass_npos(k), sizeof(long long), cudaMemcpyDeviceToHost,
-                                     c->stream));
-            CBP_CUDA(cudaStreamSynchronize(c->stream));
+            const long long npos2 = npos[k];
             const long long nd = map_diag_rows(npos2);
             const size_t nb = (size_t)map_bands(Lq);
             const long long alnstride = align_up(npos2 + (long long)np * Lq, 32);
@@ -1075,8 +1149,6 @@ void process_queries(cbp_context* c, size_t nq, const size_t* qlens, char* const
                 c->last_map_p0 = s.p0;
                 c->last_map_pass_idx = mp.pass_idx;
                 c->last_map_pass_dst = mp.pass_dst;
-                CBP_CUDA(cudaMemcpyAsync(&c->h_maperr, c->maperr.p, sizeof(int), cudaMemcpyDeviceToHost,
-                                         c->stream));
                 c->launches += 2;
                 c->stage_launches[4] += 2;
             } else {
@@ -1094,22 +1166,74 @@ void process_queries(cbp_context* c, size_t nq, const size_t* qlens, char* const
                                            c->hitkeys.as<uint64_t>() + k * keycap, c->hitcnt.as<int>() + k,
                                            c->stream);
             c->stage_launches[5] += 1;
+            // the results of the one slab are complete: the hit order too
+            const bool one = slabs.size() == 1;
+            if (one) {
+                CBP_CUDA(cudaEventRecord(c->ev[8], c->stream));
+                const int nl = launch_hit_sort(c->hitkeys.as<uint64_t>() + k * keycap, np, c->stream);
+                CBP_CUDA(cudaEventRecord(c->ev[9], c->stream));
+                c->launches += nl;
+                c->stage_launches[5] += nl;
+            }
             const size_t off = r.h_recs.size();
+            const size_t recbytes = (size_t)np * kRecFloats * sizeof(float);
             r.h_recs.resize(off + (size_t)np * kRecFloats);
-            CBP_CUDA(cudaMemcpyAsync(r.h_recs.data() + off, c->hitrecs.p, (size_t)np * kRecFloats * sizeof(float),
-                                     cudaMemcpyDeviceToHost, c->stream));
             // this slab's alignment rows go to the running offset of
             // the whole result (slot of pair K at newDst + K*Lq)
             const long long shift = r.base_len + r.base_npass * (long long)Lq;
             const long long slablen = npos2 + (long long)np * Lq;
-            for (int row = 0; row < 5; row++) {
-                r.h_alns[row].resize((size_t)(shift + slablen), 0);
-                CBP_CUDA(cudaMemcpyAsync(r.h_alns[row].data() + shift, c->alnbuf.as<char>() + (size_t)row * alnstride,
-                                         (size_t)slablen, cudaMemcpyDeviceToHost, c->stream));
+            for (int row = 0; row < 5; row++) r.h_alns[row].resize((size_t)(shift + slablen), 0);
+            // staged: flags, keys, records, rows
+            const size_t keybytes = one ? (size_t)np * sizeof(uint64_t) : 0;
+            const size_t small = 16 + keybytes + recbytes;
+            const bool staged = small + 5 * (size_t)slablen <= kMaxStaged;
+            c->rpin.reserve(16 + (staged ? small + 5 * (size_t)slablen : 0));
+            char* const pin = c->rpin.as<char>();
+            int* const pflags = reinterpret_cast<int*>(pin);
+            pflags[0] = pflags[1] = 0;
+            if (c->opt.mapaln)
+                CBP_CUDA(cudaMemcpyAsync(pflags, c->maperr.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+            if (one)
+                CBP_CUDA(cudaMemcpyAsync(pflags + 1, c->hitcnt.as<int>() + k, sizeof(int), cudaMemcpyDeviceToHost,
+                                         c->stream));
+            std::vector<uint64_t> keys;
+            if (staged) {
+                if (one)
+                    CBP_CUDA(cudaMemcpyAsync(pin + 16, c->hitkeys.as<uint64_t>() + k * keycap, keybytes,
+                                             cudaMemcpyDeviceToHost, c->stream));
+                CBP_CUDA(cudaMemcpyAsync(pin + 16 + keybytes, c->hitrecs.p, recbytes, cudaMemcpyDeviceToHost,
+                                         c->stream));
+                CBP_CUDA(cudaMemcpy2DAsync(pin + small, (size_t)slablen, c->alnbuf.p, (size_t)alnstride,
+                                           (size_t)slablen, 5, cudaMemcpyDeviceToHost, c->stream));
+            } else {
+                keys.resize(one ? (size_t)np : 0);
+                if (one)
+                    CBP_CUDA(cudaMemcpyAsync(keys.data(), c->hitkeys.as<uint64_t>() + k * keycap, keybytes,
+                                             cudaMemcpyDeviceToHost, c->stream));
+                CBP_CUDA(cudaMemcpyAsync(r.h_recs.data() + off, c->hitrecs.p, recbytes, cudaMemcpyDeviceToHost,
+                                         c->stream));
+                for (int row = 0; row < 5; row++)
+                    CBP_CUDA(cudaMemcpyAsync(r.h_alns[row].data() + shift, c->alnbuf.as<char>() + (size_t)row * alnstride,
+                                             (size_t)slablen, cudaMemcpyDeviceToHost, c->stream));
             }
             CBP_CUDA(cudaStreamSynchronize(c->stream));
+            c->h_maperr = pflags[0];
             if (c->opt.mapaln && c->h_maperr)
                 throw Error(CBP_ERR_CUDA, "MAP realignment: a wait between the warps of a pair timed out");
+            if (staged) {
+                std::memcpy(r.h_recs.data() + off, pin + 16 + keybytes, recbytes);
+                for (int row = 0; row < 5; row++)
+                    std::memcpy(r.h_alns[row].data() + shift, pin + small + (size_t)row * slablen, (size_t)slablen);
+            }
+            if (one) {
+                const int nrep = pflags[1];
+                if (nrep < 0 || nrep > np) throw Error(CBP_ERR_CUDA, "hit order: inconsistent count");
+                const uint64_t* kp = staged ? reinterpret_cast<const uint64_t*>(pin + 16) : keys.data();
+                r.h_order.resize((size_t)nrep);
+                for (int i = 0; i < nrep; i++) r.h_order[i] = (int32_t)(uint32_t)kp[i];
+                CBP_CUDA(cudaEventElapsedTime(&ms, c->ev[8], c->ev[9]));
+                c->stage_ms[5] += ms;
+            }
             CBP_CUDA(cudaEventElapsedTime(&ms, c->ev[4], c->ev[5]));
             c->stage_ms[3] += ms;
             CBP_CUDA(cudaEventElapsedTime(&ms, c->ev[6], c->ev[7]));
@@ -1130,7 +1254,7 @@ void process_queries(cbp_context* c, size_t nq, const size_t* qlens, char* const
     // over the keys of all its records; the reported ones come first
     for (size_t k = 0; k < nq; k++) {
         QueryResult& r = res[k];
-        if (r.base_npass <= 0) continue;
+        if (r.base_npass <= 0 || slabs.size() == 1) continue;   // one slab: done with its results
         uint64_t* keys_d = c->hitkeys.as<uint64_t>() + k * keycap;
         CBP_CUDA(cudaEventRecord(c->ev[4], c->stream));
         const int nl = launch_hit_sort(keys_d, r.base_npass, c->stream);
@@ -1250,6 +1374,7 @@ int cbp_destroy(cbp_context* c)
     c->sstab.release();
     c->dmstab.release();
     for (DevBuf* b : {&c->tcq, &c->tcerr}) b->release();
+    for (PinBuf* b : {&c->qpin, &c->cpin, &c->rpin}) b->release();
     for (auto& e : c->ev)
         if (e) cudaEventDestroy(e);
     if (c->stream) cudaStreamDestroy(c->stream);
