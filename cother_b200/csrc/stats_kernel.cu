@@ -545,14 +545,32 @@ stats_kernel(const StatsArgs a)
     //    (src/libmycu/cuss/CuBatchSS_dynplm.cu:77-180)
     for (int i = tid; i < NSC; i += kThreads) cnt[i] = 0;
     __syncthreads();
-    const long long ncell = (long long)Lq * Ld;
-    for (long long idx = tid; idx < ncell; idx += kThreads) {
-        const int r = (int)(idx / Ld), c = (int)(idx - (long long)r * Ld);
-        if (a.x_uninf && (a.qaa[r] == 'X' || a.db.aa[pstart + c] == 'X')) continue;
-        float s = a.scores[(long long)r * a.ld + colb + c];
-        s = s < -10.0f ? -10.0f : (s > 10.0f ? 10.0f : s);
-        const int bin = (int)rintf(s * 32.0f) + 320;
-        atomicAdd(&cnt[bin], 1);
+    // a warp takes every NS-th row, eight of its columns a lane in flight (one
+    // cell at a time with its row and column by division, a pair of 1,500 x
+    // 1,400 took 1.2 ms)
+    constexpr int kInFlight = 8;
+    for (int r = y; r < Lq; r += NS) {
+        if (a.x_uninf && a.qaa[r] == 'X') continue;
+        const float* __restrict__ S = a.scores + (long long)r * a.ld + colb;
+        const int8_t* __restrict__ aa = a.db.aa + pstart;
+        for (int c0 = x; c0 < Ld; c0 += 32 * kInFlight) {
+            float v[kInFlight];
+            bool in[kInFlight];
+#pragma unroll
+            for (int i = 0; i < kInFlight; i++) {
+                const int c = c0 + 32 * i;
+                in[i] = c < Ld && !(a.x_uninf && aa[c] == 'X');
+                v[i] = c < Ld ? S[c] : 0.0f;
+            }
+#pragma unroll
+            for (int i = 0; i < kInFlight; i++) {
+                if (!in[i]) continue;
+                float s = v[i];
+                s = s < -10.0f ? -10.0f : (s > 10.0f ? 10.0f : s);
+                const int bin = (int)rintf(s * 32.0f) + 320;
+                atomicAdd(&cnt[bin], 1);
+            }
+        }
     }
     __syncthreads();
 
