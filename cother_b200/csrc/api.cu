@@ -202,7 +202,7 @@ constexpr int kScoreRowsCand[kScoreCandidates] = {16, 8, 32, 16, 16};
 constexpr int kWindowCand[kScoreCandidates] = {1024, 1024, 1024, 256, 4096};
 constexpr int kDpWarpsCand[kDpCandidates] = {2, 1};
 constexpr int kPreferredScoreCand = 0;     // 16 rows, window 1,024
-constexpr long long kTuneCells = 2 << 20;  // cells of a sample
+constexpr long long kTuneCells = 1 << 20;  // cells of a sample
 constexpr float kTuneMargin = 0.015f;      // a candidate must be this much faster to replace it
 struct Tuning {
     int rows = 16, window = kOrderWindow, dp_warps = 2;
@@ -620,11 +620,11 @@ std::vector<Slab> plan_slabs(const cbp_context* c, int Lq)
 
 // The tuner: on the first slab of a query-length bin, time each candidate
 // kernel variant on a sample of the slab (its first profiles, up to 32,768
-// positions and about two million cells, all query rows) and keep the fastest.
-// Two million cells are three waves of the score kernel's blocks; the twelve
-// timed launches on them take about as long as searching 25 million cells,
-// where 32,768 positions made a first search against 200,000 positions four
-// times as long as the next. Every variant computes
+// positions and about a million cells, all query rows) and keep the fastest. A
+// million cells are two waves of the score kernel's blocks; the twelve timed
+// launches on them take about as long as searching 12 million cells, where
+// 32,768 positions made a first search against 200,000 positions four times as
+// long as the next. Every variant computes
 // the same cells, so the choice changes the time, never a result; the
 // sample's outputs are overwritten by the slab's own launches.
 void tune_kernels(cbp_context* c, const ScoreArgs& base, int p0, int p1, Tuning& t)
