@@ -18,11 +18,11 @@
 //    anti-diagonals (forward and MAP DP: top-down, left to right; backward:
 //    bottom-up, right to left), lane t on row r0+t, neighbours exchanged by
 //    shuffles. Warp w takes bands w, w+W, ..., so W bands are in flight at
-//    once, each running about three 32-column chunks behind the band it
-//    depends on: the dependence is the band edge (the states of the
-//    neighbouring band's last row), which the edge lane writes to a
-//    per-warp strip in global memory and publishes chunk by chunk through
-//    a counter in shared memory. Producers never wait for consumers, so
+//    once, each running 68 steps behind the band it depends on: the
+//    dependence is the band edge (the states of the neighbouring band's
+//    last row), which the edge lane writes to a strip in global memory and
+//    publishes chunk by chunk (32 columns) through a counter in shared
+//    memory. Producers never wait for consumers, so
 //    the waits form a chain that ends at the first band.
 // What bounds map_kernel is the latency of a warp's step (about 550 cycles
 // forward and backward: some 175 instructions, one warp to a scheduler), so
@@ -50,6 +50,7 @@ namespace {
 constexpr unsigned kFull = 0xffffffffu;
 constexpr float kLogP0 = -99.0f;
 constexpr float kLogSpMin = -8.7336545e+01f;
+constexpr int kSMs = 148;
 constexpr int kRows = 8;                 // diagonal rows prefetched per lane
 constexpr int kScoreWarps = 4;           // warps per block of map_scores_kernel
 constexpr long long kWaitCycles = 4000000000LL;   // about 2 s: a wait between warps gives up
@@ -398,7 +399,41 @@ __device__ __forceinline__ void run_steps(int s0, int s1, bool inside, Step&& st
     }
 }
 
+// Steps s0 .. s1-1 of a band (a chunk: 32, or fewer at its end), ahead() after
+// kEdgeAhead of them. kMany: one copy of the steps' code, in groups of four.
+// With a block or two on every SM, their warps in different passes, the steps'
+// instructions no longer stay in the instruction cache (2.2 warps a cycle and
+// scheduler waited for one, with 30 % of the cycles issuing): 400 x 494 pairs
+// 5.7 ms, against 6.9 with the two parts inlined apart, which is faster for few
+// pairs (400 x 500 profiles, 5 pairs: 2.19 ms against 2.32).
+template <bool kMany, class Step, class Ahead>
+__device__ __forceinline__ void run_chunk(int s0, int s1, bool inside, Step&& step, Ahead&& ahead)
+{
+    if constexpr (!kMany) {
+        const int sm = min(s0 + kEdgeAhead, s1);
+        run_steps(s0, sm, inside, step);
+        ahead();
+        run_steps(sm, s1, inside, step);
+    } else {
+        constexpr int kGroup = 4;
+        static_assert(kEdgeAhead % kGroup == 0, "");
+#pragma unroll 1
+        for (int s = s0; s < s0 + 32; s += kGroup) {
+            if (s == s0 + kEdgeAhead) ahead();
+            if (inside) {
+#pragma unroll
+                for (int i = 0; i < kGroup; i++) step(s + i, std::integral_constant<bool, false>());
+            } else {
+                const int se = min(s + kGroup, s1);
+#pragma unroll 1
+                for (int i = s; i < se; i++) step(i, std::integral_constant<bool, true>());
+            }
+        }
+    }
+}
+
 // ---------------- forward (fwd.cu:260-400); boundary MM 0, others -99
+template <bool kMany>
 __device__ __forceinline__ float forward_pass(const MapArgs& a, const Pair& q, BlockShared& sh,
                                               WarpStage& st, int W, int w, int nb)
 {
@@ -486,10 +521,8 @@ __device__ __forceinline__ float forward_pass(const MapArgs& a, const Pair& q, B
                 load_trn(tr, dtr, NT, Ld, J + 2, false, lane);
                 if (lane == 31 && J >= 2) publish(sh, w, e.obase + J - 1);
             }
-            const int sm = min(s0 + kEdgeAhead, s1);
-            run_steps(s0, sm, J > 0 && s1 <= Ld, step);
-            edge_load_next<5>(sh, e, Ld, er, J, a.err, lane);
-            run_steps(sm, s1, J > 0 && s1 <= Ld, step);
+            run_chunk<kMany>(s0, s1, J > 0 && s1 <= Ld, step,
+                             [&] { edge_load_next<5>(sh, e, Ld, er, J, a.err, lane); });
         }
         cp_wait<0>();
         if (lane == 31) publish(sh, w, e.obase + e.nce);
@@ -502,6 +535,7 @@ __device__ __forceinline__ float forward_pass(const MapArgs& a, const Pair& q, B
 // left; lane t at step s is at column Ld-1-s+(31-t), all lanes on
 // diagonal row Ld+30-s. The score of the diagonal successor (r+1, c+1)
 // reaches lane t from lane t+1 two steps after lane t+1 was there.
+template <bool kMany>
 __device__ __forceinline__ void backward_pass(const MapArgs& a, const Pair& q, BlockShared& sh,
                                               WarpStage& st, int W, int w, int nb)
 {
@@ -609,10 +643,8 @@ __device__ __forceinline__ void backward_pass(const MapArgs& a, const Pair& q, B
                 load_trn(tr, dtr, NT, Ld, J + 2, true, lane);
                 if (lane == 0 && J >= 2) publish(sh, w, e.obase + J - 1);
             }
-            const int sm = min(s0 + kEdgeAhead, s1);
-            run_steps(s0, sm, J > 0 && s1 <= Ld, step);
-            edge_load_next<6>(sh, e, Ld, er, J, a.err, lane);
-            run_steps(sm, s1, J > 0 && s1 <= Ld, step);
+            run_chunk<kMany>(s0, s1, J > 0 && s1 <= Ld, step,
+                             [&] { edge_load_next<6>(sh, e, Ld, er, J, a.err, lane); });
         }
         cp_wait<0>();
         if (lane == 0) publish(sh, w, e.obase + e.nce);
@@ -632,6 +664,7 @@ __device__ __forceinline__ bool better(float v, int r, int c, const Best& b)
     return b.v < v || (b.v == v && (r < b.r || (r == b.r && c < b.c)));
 }
 
+template <bool kMany>
 __device__ __forceinline__ Best map_pass(const MapArgs& a, const Pair& q, BlockShared& sh,
                                          WarpStage& st, int W, int w, int nb, float logz)
 {
@@ -696,10 +729,8 @@ __device__ __forceinline__ Best map_pass(const MapArgs& a, const Pair& q, BlockS
                 __syncwarp();
                 if (lane == 31 && J >= 2) publish(sh, w, e.obase + J - 1);
             }
-            const int sm = min(s0 + kEdgeAhead, s1);
-            run_steps(s0, sm, J > 0 && s1 <= Ld, step);
-            edge_load_next<1>(sh, e, Ld, er, J, a.err, lane);
-            run_steps(sm, s1, J > 0 && s1 <= Ld, step);
+            run_chunk<kMany>(s0, s1, J > 0 && s1 <= Ld, step,
+                             [&] { edge_load_next<1>(sh, e, Ld, er, J, a.err, lane); });
         }
         cp_wait<0>();
         if (lane == 31) publish(sh, w, e.obase + e.nce);
@@ -708,7 +739,9 @@ __device__ __forceinline__ Best map_pass(const MapArgs& a, const Pair& q, BlockS
     return best;
 }
 
-__global__ void __launch_bounds__(32 * kMapMaxWarps)
+// kMany: see run_chunk() and map_pair_warps()
+template <bool kMany>
+__global__ void __launch_bounds__(32 * (kMany ? kMapMaxWarps / 2 : kMapMaxWarps), kMany ? 2 : 1)
 map_kernel(const MapArgs a, int nb)
 {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -730,7 +763,7 @@ map_kernel(const MapArgs a, int nb)
     __syncthreads();
     WarpStage& st = stages[w];
 
-    float maxlp = forward_pass(a, q, sh, st, W, w, nb);
+    float maxlp = forward_pass<kMany>(a, q, sh, st, W, w, nb);
     for (int o = 16; o >= 1; o >>= 1) maxlp = hmax(maxlp, __shfl_xor_sync(kFull, maxlp, o));
     if (lane == 0) sh.fmax[w] = maxlp;
     __syncthreads();
@@ -764,12 +797,12 @@ map_kernel(const MapArgs a, int nb)
     __syncthreads();
     const float logz = sh.logz;
 
-    backward_pass(a, q, sh, st, W, w, nb);
+    backward_pass<kMany>(a, q, sh, st, W, w, nb);
     __syncthreads();
     if (threadIdx.x < kMapMaxWarps) sh.prog[threadIdx.x] = 0;
     __syncthreads();
 
-    Best best = map_pass(a, q, sh, st, W, w, nb, logz);
+    Best best = map_pass<kMany>(a, q, sh, st, W, w, nb, logz);
     for (int o = 16; o >= 1; o >>= 1) {
         const float ov = __shfl_xor_sync(kFull, best.v, o);
         const int orr = __shfl_xor_sync(kFull, best.r, o), oc = __shfl_xor_sync(kFull, best.c, o);
@@ -990,7 +1023,7 @@ void launch_aln_final(const MapArgs& a, const uint8_t* btck1, const float* maxsc
 // every SM, 8: two such blocks share an SM.
 static int map_pair_warps(int npass, int nb)
 {
-    const int most = npass <= 148 ? kMapMaxWarps : kMapMaxWarps / 2;
+    const int most = npass <= kSMs ? kMapMaxWarps : kMapMaxWarps / 2;
     return nb < most ? nb : most;
 }
 
@@ -1006,8 +1039,12 @@ void launch_map(const MapArgs& a, cudaStream_t stream)
     CBP_CHECK_LAUNCH();
     const int W = map_pair_warps(a.npass, nb);
     const size_t smem = kSharedHead + (size_t)W * sizeof(WarpStage) + (size_t)nb * sizeof(float);
-    CBP_CUDA(cudaFuncSetAttribute(map_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    map_kernel<<<a.npass, 32 * W, smem, stream>>>(a, nb);
+    // one copy of the steps' code from about one and a half pairs an SM (400:
+    // 192 pairs 2.66 ms without and 2.79 with, 482 pairs 7.6 and 7.0; 1,000: 276
+    // pairs 7.3 and 7.0)
+    const auto kernel = a.npass > 3 * kSMs / 2 ? map_kernel<true> : map_kernel<false>;
+    CBP_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kernel<<<a.npass, 32 * W, smem, stream>>>(a, nb);
     CBP_CHECK_LAUNCH();
 }
 

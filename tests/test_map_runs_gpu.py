@@ -21,3 +21,18 @@ def test_profile_lengths_around_chunks(oracle_lib, ss_table, Lq):
         assert _check_map(bp, oracle_lib, q, db, minpp=0.05, logethld=1e9) >= 4
     finally:
         bp.close()
+
+
+@pytest.mark.parametrize("Lq", [33, 97, 290])
+def test_many_pairs(oracle_lib, ss_table, Lq):
+    """More pairs than one and a half an SM take the steps in groups of four:
+    chunks that end inside and between groups, and more bands than warps."""
+    from cother_b200 import synth
+    q = synth.make_profiles([Lq], 1300 + Lq, True)
+    db = synth.make_profiles([*range(26, 38), *range(58, 70), 93, 96, 97, 100] * 12, 1400 + Lq, False)
+    synth.plant_homologs(q, db, 1.0, seed=Lq)
+    bp = _search(q, db, ss_table, thld=-1.0, logethld=1e9, minpp=0.05, all_codes=1)
+    try:
+        assert _check_map(bp, oracle_lib, q, db, minpp=0.05, logethld=1e9) > 222
+    finally:
+        bp.close()
