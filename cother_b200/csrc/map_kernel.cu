@@ -76,10 +76,13 @@ __device__ __forceinline__ float fexp_neg(float a)
     const uint32_t x = __float_as_uint(__fmaf_rn(12102203.16f, a, 1064631197.0f)) * 64u + 0xa0000000u;
     return -16.0f < a ? __uint_as_float(x) : 0.0f;
 }
-// log(exp(v1) + exp(v2)): the larger one's term is fexp(0)
+// log(exp(v1) + exp(v2)): the larger one's term is fexp(0). By one comparison,
+// as hmax selects (fmaxf and fminf would drop a NaN): a NaN in v1 is the
+// result, one in v2 adds nothing.
 __device__ __forceinline__ float lse2(float v1, float v2)
 {
-    const float m = fmaxf(v1, v2), d = fminf(v1, v2) - m;
+    const bool up = v1 < v2;
+    const float m = up ? v2 : v1, d = (up ? v1 : v2) - m;
     return flog(__int_as_float(1064631168) + fexp_neg(d)) + m;
 }
 
