@@ -1337,6 +1337,7 @@ int cbp_create(int device, const cbp_options* opt, const float* ss_table, size_t
             CBP_CUDA(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
             for (auto& e : c->ev) CBP_CUDA(cudaEventCreate(&e));
             dp1_set_attributes();
+            map_set_attributes();
             tc_set_attributes();
             std::memcpy(c->sstab_h, ss_table, sizeof(c->sstab_h));
             build_dms_table(c->dmstab_h);

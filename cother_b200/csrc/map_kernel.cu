@@ -1030,6 +1030,24 @@ static int map_pair_warps(int npass, int nb)
     return nb < most ? nb : most;
 }
 
+static size_t map_shared_bytes(int W, int nb)
+{
+    return kSharedHead + (size_t)W * sizeof(WarpStage) + (size_t)nb * sizeof(float);
+}
+
+// The attribute belongs to the function on the device, which the contexts of
+// all threads share: set once to the most that any launch asks for (a query
+// has fewer than 65,536 positions), never to the need of one launch, which
+// another thread's could lower in between.
+void map_set_attributes()
+{
+    constexpr int kMostBands = 65536 / 32;
+    CBP_CUDA(cudaFuncSetAttribute(map_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)map_shared_bytes(kMapMaxWarps, kMostBands)));
+    CBP_CUDA(cudaFuncSetAttribute(map_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)map_shared_bytes(kMapMaxWarps / 2, kMostBands)));
+}
+
 void launch_map(const MapArgs& a, cudaStream_t stream)
 {
     if (a.npass <= 0) return;
@@ -1041,12 +1059,11 @@ void launch_map(const MapArgs& a, cudaStream_t stream)
     map_scores_kernel<<<sgrid, 32 * kScoreWarps, 0, stream>>>(a, nb);
     CBP_CHECK_LAUNCH();
     const int W = map_pair_warps(a.npass, nb);
-    const size_t smem = kSharedHead + (size_t)W * sizeof(WarpStage) + (size_t)nb * sizeof(float);
     // one copy of the steps' code from about one and a half pairs an SM (400:
     // 192 pairs 2.66 ms without and 2.79 with, 482 pairs 7.6 and 7.0; 1,000: 276
     // pairs 7.3 and 7.0)
     const auto kernel = a.npass > 3 * kSMs / 2 ? map_kernel<true> : map_kernel<false>;
-    CBP_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const size_t smem = map_shared_bytes(W, nb);
     kernel<<<a.npass, 32 * W, smem, stream>>>(a, nb);
     CBP_CHECK_LAUNCH();
 }

@@ -55,6 +55,9 @@ inline long long map_strip_floats(long long npos2)
     return (long long)kMapStrips * kMapEdgeFields * npos2;
 }
 
+// Per device, before the first launch_map (and outside any stream capture): the
+// shared-memory opt-in of the MAP kernel.
+void map_set_attributes();
 // zeroes sg and bt, then realigns every pair of the pass list
 void launch_map(const MapArgs& a, cudaStream_t stream);
 
