@@ -402,17 +402,20 @@ __device__ __forceinline__ void run_steps(int s0, int s1, bool inside, Step&& st
     }
 }
 
+// How the steps of a chunk are laid out in code, by how many warps in different
+// passes share an SM's instruction cache (map_step_code()).
+enum StepCode {
+    kApart,     // the two parts of a chunk inlined apart, with and without checks: the shortest chain
+    kGroups,    // one copy, in groups of four without checks, and one with checks
+    kOne        // one step, with checks
+};
+
 // Steps s0 .. s1-1 of a band (a chunk: 32, or fewer at its end), ahead() after
-// kEdgeAhead of them. kMany: one copy of the steps' code, in groups of four.
-// With a block or two on every SM, their warps in different passes, the steps'
-// instructions no longer stay in the instruction cache (2.2 warps a cycle and
-// scheduler waited for one, with 30 % of the cycles issuing): 400 x 494 pairs
-// 5.7 ms, against 6.9 with the two parts inlined apart, which is faster for few
-// pairs (400 x 500 profiles, 5 pairs: 2.19 ms against 2.32).
-template <bool kMany, class Step, class Ahead>
+// kEdgeAhead of them.
+template <StepCode kCode, class Step, class Ahead>
 __device__ __forceinline__ void run_chunk(int s0, int s1, bool inside, Step&& step, Ahead&& ahead)
 {
-    if constexpr (!kMany) {
+    if constexpr (kCode == kApart) {
         const int sm = min(s0 + kEdgeAhead, s1);
         run_steps(s0, sm, inside, step);
         ahead();
@@ -423,7 +426,7 @@ __device__ __forceinline__ void run_chunk(int s0, int s1, bool inside, Step&& st
 #pragma unroll 1
         for (int s = s0; s < s0 + 32; s += kGroup) {
             if (s == s0 + kEdgeAhead) ahead();
-            if (inside) {
+            if (kCode == kGroups && inside) {
 #pragma unroll
                 for (int i = 0; i < kGroup; i++) step(s + i, std::integral_constant<bool, false>());
             } else {
@@ -436,7 +439,7 @@ __device__ __forceinline__ void run_chunk(int s0, int s1, bool inside, Step&& st
 }
 
 // ---------------- forward (fwd.cu:260-400); boundary MM 0, others -99
-template <bool kMany>
+template <StepCode kCode>
 __device__ __forceinline__ float forward_pass(const MapArgs& a, const Pair& q, BlockShared& sh,
                                               WarpStage& st, int W, int w, int nb)
 {
@@ -524,7 +527,7 @@ __device__ __forceinline__ float forward_pass(const MapArgs& a, const Pair& q, B
                 load_trn(tr, dtr, NT, Ld, J + 2, false, lane);
                 if (lane == 31 && J >= 2) publish(sh, w, e.obase + J - 1);
             }
-            run_chunk<kMany>(s0, s1, J > 0 && s1 <= Ld, step,
+            run_chunk<kCode>(s0, s1, J > 0 && s1 <= Ld, step,
                              [&] { edge_load_next<5>(sh, e, Ld, er, J, a.err, lane); });
         }
         cp_wait<0>();
@@ -538,7 +541,7 @@ __device__ __forceinline__ float forward_pass(const MapArgs& a, const Pair& q, B
 // left; lane t at step s is at column Ld-1-s+(31-t), all lanes on
 // diagonal row Ld+30-s. The score of the diagonal successor (r+1, c+1)
 // reaches lane t from lane t+1 two steps after lane t+1 was there.
-template <bool kMany>
+template <StepCode kCode>
 __device__ __forceinline__ void backward_pass(const MapArgs& a, const Pair& q, BlockShared& sh,
                                               WarpStage& st, int W, int w, int nb)
 {
@@ -646,7 +649,7 @@ __device__ __forceinline__ void backward_pass(const MapArgs& a, const Pair& q, B
                 load_trn(tr, dtr, NT, Ld, J + 2, true, lane);
                 if (lane == 0 && J >= 2) publish(sh, w, e.obase + J - 1);
             }
-            run_chunk<kMany>(s0, s1, J > 0 && s1 <= Ld, step,
+            run_chunk<kCode>(s0, s1, J > 0 && s1 <= Ld, step,
                              [&] { edge_load_next<6>(sh, e, Ld, er, J, a.err, lane); });
         }
         cp_wait<0>();
@@ -667,7 +670,7 @@ __device__ __forceinline__ bool better(float v, int r, int c, const Best& b)
     return b.v < v || (b.v == v && (r < b.r || (r == b.r && c < b.c)));
 }
 
-template <bool kMany>
+template <StepCode kCode>
 __device__ __forceinline__ Best map_pass(const MapArgs& a, const Pair& q, BlockShared& sh,
                                          WarpStage& st, int W, int w, int nb, float logz)
 {
@@ -732,7 +735,7 @@ __device__ __forceinline__ Best map_pass(const MapArgs& a, const Pair& q, BlockS
                 __syncwarp();
                 if (lane == 31 && J >= 2) publish(sh, w, e.obase + J - 1);
             }
-            run_chunk<kMany>(s0, s1, J > 0 && s1 <= Ld, step,
+            run_chunk<kCode>(s0, s1, J > 0 && s1 <= Ld, step,
                              [&] { edge_load_next<1>(sh, e, Ld, er, J, a.err, lane); });
         }
         cp_wait<0>();
@@ -742,9 +745,10 @@ __device__ __forceinline__ Best map_pass(const MapArgs& a, const Pair& q, BlockS
     return best;
 }
 
-// kMany: see run_chunk() and map_pair_warps()
-template <bool kMany>
-__global__ void __launch_bounds__(32 * (kMany ? kMapMaxWarps / 2 : kMapMaxWarps), kMany ? 2 : 1)
+// kCode: see map_step_code(); with more pairs than map_pair_warps() gives all
+// warps, two blocks share an SM
+template <StepCode kCode>
+__global__ void __launch_bounds__(32 * (kCode == kApart ? kMapMaxWarps : kMapMaxWarps / 2), kCode == kApart ? 1 : 2)
 map_kernel(const MapArgs a, int nb)
 {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -766,7 +770,7 @@ map_kernel(const MapArgs a, int nb)
     __syncthreads();
     WarpStage& st = stages[w];
 
-    float maxlp = forward_pass<kMany>(a, q, sh, st, W, w, nb);
+    float maxlp = forward_pass<kCode>(a, q, sh, st, W, w, nb);
     for (int o = 16; o >= 1; o >>= 1) maxlp = hmax(maxlp, __shfl_xor_sync(kFull, maxlp, o));
     if (lane == 0) sh.fmax[w] = maxlp;
     __syncthreads();
@@ -800,12 +804,12 @@ map_kernel(const MapArgs a, int nb)
     __syncthreads();
     const float logz = sh.logz;
 
-    backward_pass<kMany>(a, q, sh, st, W, w, nb);
+    backward_pass<kCode>(a, q, sh, st, W, w, nb);
     __syncthreads();
     if (threadIdx.x < kMapMaxWarps) sh.prog[threadIdx.x] = 0;
     __syncthreads();
 
-    Best best = map_pass<kMany>(a, q, sh, st, W, w, nb, logz);
+    Best best = map_pass<kCode>(a, q, sh, st, W, w, nb, logz);
     for (int o = 16; o >= 1; o >>= 1) {
         const float ov = __shfl_xor_sync(kFull, best.v, o);
         const int orr = __shfl_xor_sync(kFull, best.r, o), oc = __shfl_xor_sync(kFull, best.c, o);
@@ -1030,6 +1034,21 @@ static int map_pair_warps(int npass, int nb)
     return nb < most ? nb : most;
 }
 
+// The layout of the steps' code. The warps of an SM are in different passes, and
+// their steps' instructions must stay in its instruction cache: with 494 pairs
+// of 400 and the parts inlined apart, 2.2 warps a cycle and scheduler waited for
+// an instruction with 30 % of the cycles issuing. The lines lie where the
+// measured times of the MAP stage cross (Lq x pairs of the 220-median length
+// law: ms of kApart / kGroups / kOne): 400 x 120:
+// 1.78 / - / 1.92; 100 x 250: 1.49 / 1.51 / 1.55; 400 x 250: 3.56 / 3.41 / 3.51;
+// 400 x 450: - / 4.26 / 4.28; 64 x 500: 1.35 / 1.27 / 1.30; 64 x 600: - / 1.35 /
+// 1.35; 250 x 600: - / 3.24 / 3.15; 400 x 800: - / 6.92 / 6.61; 200 x 2,000: 14.5 /
+// 9.94 / 8.60; 64 x 2,000: 4.54 / 3.45 / 2.72.
+static StepCode map_step_code(int npass)
+{
+    return npass <= 3 * kSMs / 2 ? kApart : npass < 4 * kSMs ? kGroups : kOne;
+}
+
 static size_t map_shared_bytes(int W, int nb)
 {
     return kSharedHead + (size_t)W * sizeof(WarpStage) + (size_t)nb * sizeof(float);
@@ -1042,10 +1061,13 @@ static size_t map_shared_bytes(int W, int nb)
 void map_set_attributes()
 {
     constexpr int kMostBands = 65536 / 32;
-    CBP_CUDA(cudaFuncSetAttribute(map_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)map_shared_bytes(kMapMaxWarps, kMostBands)));
-    CBP_CUDA(cudaFuncSetAttribute(map_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)map_shared_bytes(kMapMaxWarps / 2, kMostBands)));
+    const auto set = [](auto kernel, int W) {
+        CBP_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)map_shared_bytes(W, kMostBands)));
+    };
+    set(map_kernel<kApart>, kMapMaxWarps);
+    set(map_kernel<kGroups>, kMapMaxWarps / 2);
+    set(map_kernel<kOne>, kMapMaxWarps / 2);
 }
 
 void launch_map(const MapArgs& a, cudaStream_t stream)
@@ -1059,10 +1081,8 @@ void launch_map(const MapArgs& a, cudaStream_t stream)
     map_scores_kernel<<<sgrid, 32 * kScoreWarps, 0, stream>>>(a, nb);
     CBP_CHECK_LAUNCH();
     const int W = map_pair_warps(a.npass, nb);
-    // one copy of the steps' code from about one and a half pairs an SM (400:
-    // 192 pairs 2.66 ms without and 2.79 with, 482 pairs 7.6 and 7.0; 1,000: 276
-    // pairs 7.3 and 7.0)
-    const auto kernel = a.npass > 3 * kSMs / 2 ? map_kernel<true> : map_kernel<false>;
+    const StepCode code = map_step_code(a.npass);
+    const auto kernel = code == kApart ? map_kernel<kApart> : code == kGroups ? map_kernel<kGroups> : map_kernel<kOne>;
     const size_t smem = map_shared_bytes(W, nb);
     kernel<<<a.npass, 32 * W, smem, stream>>>(a, nb);
     CBP_CHECK_LAUNCH();
