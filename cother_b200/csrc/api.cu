@@ -134,24 +134,13 @@ struct DevBuf {
     template <class T> T* as() const { return static_cast<T*>(p); }
 };
 
-// A page-locked host buffer that only grows: what a small upload or read-back
-// is staged in, so that it is one asynchronous copy.
-struct PinBuf {
-    void* p = nullptr;
-    size_t bytes = 0;
-    void reserve(size_t n) {
-        if (n <= bytes) return;
-        release();
-        CBP_CUDA(cudaHostAlloc(&p, n, cudaHostAllocDefault));
-        bytes = n;
-    }
-    void release() {
-        if (p) cudaFreeHost(p);
-        p = nullptr; bytes = 0;
-    }
-    template <class T> T* as() const { return static_cast<T*>(p); }
-};
-constexpr size_t kMaxStaged = 4u << 20;   // larger copies go straight to their places
+// Small profile sets (queries) are packed in pageable host memory, to go up in
+// one copy, and the results of a search come down in one. Page-locked memory
+// is no faster at these sizes (150 KB up: 20 us against 21 with the packing;
+// 10 KB down: 17 against 15), but an allocation of it takes 0.4 to 3 ms, and
+// three of them made a first search of 8 x 8 positions 3.0 ms long instead of
+// 1.2.
+constexpr size_t kMaxPacked = 4u << 20;   // larger sets go straight to their places
 
 // Device copy of a packed profile set.
 struct ProfilesStore {
@@ -220,7 +209,15 @@ struct QueryResult {
     unsigned long long searchspace = 0;
     size_t delta_length = 0;
     std::vector<float> h_recs;       // hit records, all slabs
-    std::vector<char> h_alns[5];     // alignment rows, all slabs
+    std::vector<char> h_alns[5];     // alignment rows, of several slabs
+    std::vector<char> h_block;       // of one slab: its results as the device holds them
+    bool one_slab = false;
+    size_t block_rows = 0, block_stride = 0, block_len = 0;   // the alignment rows in the block
+    const char* row(int i) const
+    {
+        return one_slab ? h_block.data() + block_rows + (size_t)i * block_stride : h_alns[i].data();
+    }
+    size_t row_length() const { return one_slab ? block_len : h_alns[0].size(); }
     std::vector<int32_t> h_order;    // reported hits in the finalizer's order (sorted on the device)
     long long base_len = 0, base_npass = 0;   // running phase-2 offsets over slabs
     long long last_npos2 = 0;
@@ -262,7 +259,8 @@ struct cbp_context {
     float cvs_key_first = 0.f, cvs_key_last = 0.f;
     // working buffers
     DevBuf scores, modscores, btck, bandbuf, colorder, dpmax, dpcoords, dprecs, passidx, passdst, passcnt;
-    DevBuf hitrecs, statrecs, cs2, fb2, sg2, bt2, strip2, maperr, alnbuf, dp1err;
+    DevBuf statrecs, cs2, fb2, sg2, bt2, strip2;
+    DevBuf results;            // of the query in hand: hit records, the MAP stage's flag, alignment rows
     DevBuf hitkeys, hitcnt;    // sort keys of all records of a query, reported count
     DevBuf fits;               // the precision forms: FP64 and FP32 parameter fits per passed pair
     DevBuf qtrn;               // batches: each query's transitions as [7][Lq+1]
@@ -298,7 +296,7 @@ struct cbp_context {
     uint64_t graph_launches = 0;
     // instrumentation
     cudaEvent_t ev[10]{};
-    PinBuf qpin, cpin, rpin;        // staging of the queries, the pass counts, the results
+    std::vector<char> qpack;        // packed queries
     float stage_ms[6] = {0, 0, 0, 0, 0, 0};
     uint64_t launches = 0;
     uint64_t stage_launches[6] = {0, 0, 0, 0, 0, 0};
@@ -345,11 +343,12 @@ size_t field_bytes(char* const* beg, char* const* end, int f)
 
 // Repack 181 SoA host fields into the device layout (layout.h) and upload.
 // Upload a packed profile set. With `with_cv` the context-vector fields
-// (pmv2DCVentrs.., pmv2DCVprior, pmv2DCVnorm2) are uploaded too. With `pin` a
-// small set (queries) is packed there and goes up in one asynchronous copy
-// (its 60-odd copies from pageable memory and their wait took about 0.2 ms).
+// (pmv2DCVentrs.., pmv2DCVprior, pmv2DCVnorm2) are uploaded too. With `pack` a
+// small set (queries) is packed there and goes up in one copy (60-odd copies
+// and their wait took about 0.2 ms); the caller keeps the buffer until the
+// stream has been waited for.
 void upload_profiles(ProfilesStore& st, char* const* beg, char* const* end, cudaStream_t stream,
-                     bool with_cv, PinBuf* pin = nullptr)
+                     bool with_cv, std::vector<char>* pack = nullptr)
 {
     if (!beg || !end) throw Error(CBP_ERR_ARG, "null field tables");
     const size_t P = field_bytes(beg, end, fLen) / sizeof(int);
@@ -489,18 +488,18 @@ void upload_profiles(ProfilesStore& st, char* const* beg, char* const* end, cuda
         t.base = total;
         total += (size_t)align_up((long long)std::max<size_t>(t.bytes, 16), 256);
     }
-    const bool small = pin && total <= kMaxStaged;
+    const bool small = pack && total <= kMaxPacked;
     if (small) {
-        pin->reserve(total);
+        if (pack->size() < total) pack->resize(total);
         st.blob.reserve(total);
         for (const Part& t : parts) {
-            char* o = pin->as<char>() + t.base;
+            char* o = pack->data() + t.base;
             for (const auto& x : t.pieces) {
                 std::memcpy(o, x.first, x.second);
                 o += x.second;
             }
         }
-        CBP_CUDA(cudaMemcpyAsync(st.blob.p, pin->p, total, cudaMemcpyHostToDevice, stream));
+        CBP_CUDA(cudaMemcpyAsync(st.blob.p, pack->data(), total, cudaMemcpyHostToDevice, stream));
     } else {
         for (const Part& t : parts) {
             t.buf->reserve(std::max<size_t>(t.bytes, 16));
@@ -774,12 +773,12 @@ void process_queries(cbp_context* c, size_t nq, const size_t* qlens, char* const
                                        "(transferred by a context with CVSWGT > 0)");
     }
     if (nq == 1) {
-        upload_profiles(c->query, qbeg[0], qend[0], c->stream, c->opt.cvswgt > 0.0f, &c->qpin);
+        upload_profiles(c->query, qbeg[0], qend[0], c->stream, c->opt.cvswgt > 0.0f, &c->qpack);
         if (c->query.view.P != 1) throw Error(CBP_ERR_ARG, "the query field tables must hold one profile");
     } else {
         StackedTables t;
         stack_tables(nq, qbeg, qend, t);
-        upload_profiles(c->query, t.beg, t.end, c->stream, c->opt.cvswgt > 0.0f, &c->qpin);
+        upload_profiles(c->query, t.beg, t.end, c->stream, c->opt.cvswgt > 0.0f, &c->qpack);
     }
     const int Ltot = (int)c->query.view.N;
     std::vector<QueryResult> res(nq);
@@ -813,6 +812,9 @@ void process_queries(cbp_context* c, size_t nq, const size_t* qlens, char* const
     c->last_map_np = 0;
     for (float& m : c->stage_ms) m = 0.f;
     for (uint64_t& m : c->stage_launches) m = 0;
+    // the last call's results go; their buffers, unless large, take this call's
+    for (size_t k = 0; k < std::min(nq, c->res.size()); k++)
+        if (c->res[k].h_block.size() <= kMaxPacked) res[k].h_block.swap(c->res[k].h_block);
     c->res.clear();
     c->cur = 0;
 
@@ -833,9 +835,11 @@ void process_queries(cbp_context* c, size_t nq, const size_t* qlens, char* const
     c->dprecs.reserve(nq * maxprof * sizeof(Dp1Rec));
     c->passidx.reserve(nq * maxprof * sizeof(int));
     c->passdst.reserve(nq * maxprof * sizeof(long long));
-    c->passcnt.reserve(nq * 16);
-    c->dp1err.reserve(sizeof(int));
-    c->hitkeys.reserve(nq * keycap * sizeof(uint64_t));
+    c->passcnt.reserve(nq * 16 + sizeof(int));
+    // behind the counts of all queries, the flag of the phase-1 launches' waits
+    int* const dp1err = reinterpret_cast<int*>(c->passcnt.as<char>() + nq * 16);
+    const bool one = slabs.size() == 1;
+    if (!one) c->hitkeys.reserve(nq * keycap * sizeof(uint64_t));
     c->hitcnt.reserve(nq * sizeof(int));
     CBP_CUDA(cudaMemsetAsync(c->hitcnt.p, 0, nq * sizeof(int), c->stream));
     // each query's transitions as the kernels index them ([7][Lq+1])
@@ -885,7 +889,7 @@ void process_queries(cbp_context* c, size_t nq, const size_t* qlens, char* const
         a.dmstab = c->dmstab.as<float>();
         a.scores = c->scores.as<float>();
         a.modscores = c->modscores.as<float>();
-        a.err = c->dp1err.as<int>();   // shared with the phase-1 DP: 2 = score kernel, 1 = DP
+        a.err = dp1err;   // shared with the phase-1 DP: 2 = score kernel, 1 = DP
         // the column order only balances the DDMS loops of a warp's lanes;
         // without that term the identity keeps the stores coalesced
         a.colorder = a.ddmswgt > 0.0f ? c->colorder.as<int>() : nullptr;
@@ -943,7 +947,7 @@ void process_queries(cbp_context* c, size_t nq, const size_t* qlens, char* const
             d[k].code_thld = c->opt.all_codes ? -INFINITY : r.score_thld;
             d[k].recs = c->dprecs.as<Dp1Rec>() + k * maxprof;
             d[k].warps = tn.dp_warps;
-            d[k].err = c->dp1err.as<int>();
+            d[k].err = dp1err;
         }
         auto pass_idx = [&](size_t k) { return c->passidx.as<int>() + k * maxprof; };
         auto pass_dst = [&](size_t k) { return c->passdst.as<long long>() + k * maxprof; };
@@ -961,7 +965,7 @@ void process_queries(cbp_context* c, size_t nq, const size_t* qlens, char* const
                 else CBP_CUDA(cudaEventRecord(e, c->stream));
             };
             if (!tc) mark(c->ev[0]);
-            CBP_CUDA(cudaMemsetAsync(c->dp1err.p, 0, sizeof(int), c->stream));
+            CBP_CUDA(cudaMemsetAsync(dp1err, 0, sizeof(int), c->stream));
             if (a.colorder)
                 launch_column_order(c->db->view.dstlen, s.col0, s.ncols, a.ld, tn.window, c->colorder.as<int>(),
                                     c->stream);
@@ -1013,19 +1017,16 @@ void process_queries(cbp_context* c, size_t nq, const size_t* qlens, char* const
         c->stage_launches[0] += 2;
         c->stage_launches[1] += (uint64_t)dp_launches;
         c->stage_launches[2] += 2 * (uint64_t)nq;
-        // the pass counts and phase-2 positions of all queries, and the flag of
-        // the launches' waits
-        c->cpin.reserve(nq * 16 + sizeof(int));
-        int* const flag = reinterpret_cast<int*>(c->cpin.as<char>() + nq * 16);
-        CBP_CUDA(cudaMemcpyAsync(c->cpin.p, c->passcnt.p, nq * 16, cudaMemcpyDeviceToHost, c->stream));
-        CBP_CUDA(cudaMemcpyAsync(flag, c->dp1err.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+        // the pass counts and phase-2 positions of all queries, and the flag
+        std::vector<char> counts(nq * 16 + sizeof(int));
+        CBP_CUDA(cudaMemcpyAsync(counts.data(), c->passcnt.p, counts.size(), cudaMemcpyDeviceToHost, c->stream));
         CBP_CUDA(cudaStreamSynchronize(c->stream));
-        c->h_dp1err = *flag;
+        std::memcpy(&c->h_dp1err, counts.data() + nq * 16, sizeof(int));
         std::vector<int> npass(nq, 0);
         std::vector<long long> npos(nq, 0);
         for (size_t k = 0; k < nq; k++) {
-            std::memcpy(&npass[k], c->cpin.as<char>() + 16 * k, sizeof(int));
-            std::memcpy(&npos[k], c->cpin.as<char>() + 16 * k + 8, sizeof(long long));
+            std::memcpy(&npass[k], counts.data() + 16 * k, sizeof(int));
+            std::memcpy(&npos[k], counts.data() + 16 * k + 8, sizeof(long long));
         }
         if (c->h_dp1err == 2)
             throw Error(CBP_ERR_CUDA, "score matrix: a wait for the bulk-copied distance lists timed out");
@@ -1058,7 +1059,18 @@ void process_queries(cbp_context* c, size_t nq, const size_t* qlens, char* const
             const int Lq = r.Lq;
             const float* sc = a.scores + (long long)r.row0 * a.ld;
             // statistics and E-values of the passed pairs of this slab
-            c->hitrecs.reserve((size_t)np * kRecFloats * sizeof(float));
+            const size_t recbytes = (size_t)np * kRecFloats * sizeof(float);
+            const long long npos2 = npos[k];
+            const long long alnstride = align_up(npos2 + (long long)np * Lq, 32);
+            const size_t flagoff = (size_t)align_up((long long)recbytes, 256), rowsoff = flagoff + 256;
+            // the keys of the hit order: with several slabs, of all of them together
+            const size_t keysoff = rowsoff + (size_t)align_up(5 * alnstride, 256);
+            c->results.reserve(keysoff + (one ? (size_t)hit_sort_capacity(np) * sizeof(uint64_t) : 0));
+            uint64_t* const keys_d = one ? reinterpret_cast<uint64_t*>(c->results.as<char>() + keysoff)
+                                         : c->hitkeys.as<uint64_t>() + k * keycap;
+            float* const hitrecs = c->results.as<float>();
+            int* const maperr = reinterpret_cast<int*>(c->results.as<char>() + flagoff);
+            char* const alnbuf = c->results.as<char>() + rowsoff;
             StatsArgs st;
             st.scores = sc;
             st.ld = a.ld;
@@ -1072,7 +1084,7 @@ void process_queries(cbp_context* c, size_t nq, const size_t* qlens, char* const
             st.pass_idx = pass_idx(k);
             st.pass_dst = pass_dst(k);
             st.recs = d[k].recs;
-            st.out = c->hitrecs.as<float>();
+            st.out = hitrecs;
             st.nnweights = c->nnweights.as<float>();
             st.ssemodel = c->opt.ssemodel;
             st.searchspace = (float)r.searchspace;
@@ -1090,19 +1102,15 @@ void process_queries(cbp_context* c, size_t nq, const size_t* qlens, char* const
             launch_stats(st, np, c->stream);
             CBP_CUDA(cudaEventRecord(c->ev[5], c->stream));
             // the records as the statistics leave them (cbp_read_statistics)
-            c->statrecs.reserve((size_t)np * kRecFloats * sizeof(float));
-            CBP_CUDA(cudaMemcpyAsync(c->statrecs.p, c->hitrecs.p, (size_t)np * kRecFloats * sizeof(float),
-                                     cudaMemcpyDeviceToDevice, c->stream));
+            c->statrecs.reserve(recbytes);
+            CBP_CUDA(cudaMemcpyAsync(c->statrecs.p, hitrecs, recbytes, cudaMemcpyDeviceToDevice, c->stream));
             c->launches += 1;
             c->stage_launches[3] += 1;
 
             // phase-2 MAP realignment of the pairs within the E-value
             // threshold (in the phase-2 column space of this slab)
-            const long long npos2 = npos[k];
             const long long nd = map_diag_rows(npos2);
             const size_t nb = (size_t)map_bands(Lq);
-            const long long alnstride = align_up(npos2 + (long long)np * Lq, 32);
-            c->alnbuf.reserve(5 * (size_t)alnstride);
             MapArgs mp;
             mp.scores = sc;
             mp.modscores = a.modscores + (long long)r.row0 * a.ld;
@@ -1121,25 +1129,23 @@ void process_queries(cbp_context* c, size_t nq, const size_t* qlens, char* const
             mp.npass = np;
             mp.pass_idx = pass_idx(k);
             mp.pass_dst = pass_dst(k);
-            mp.recs = c->hitrecs.as<float>();
-            mp.alns = c->alnbuf.as<char>();
+            mp.recs = hitrecs;
+            mp.alns = alnbuf;
             mp.alnstride = alnstride;
-            CBP_CUDA(cudaMemsetAsync(c->alnbuf.p, 0, 5 * (size_t)alnstride, c->stream));
+            CBP_CUDA(cudaMemsetAsync(maperr, 0, 256 + 5 * (size_t)alnstride, c->stream));   // the flag and the rows
             if (c->opt.mapaln) {
                 c->cs2.reserve(nb * nd * 32 * sizeof(float));
                 c->fb2.reserve(nb * nd * 32 * sizeof(float));
                 c->sg2.reserve(nb * nd * sizeof(unsigned));
                 c->bt2.reserve(nb * nd * sizeof(unsigned long long));
                 c->strip2.reserve((size_t)map_strip_floats(npos2) * sizeof(float));
-                c->maperr.reserve(sizeof(int));
                 mp.nd = nd;
                 mp.cs = c->cs2.as<float>();
                 mp.fb = c->fb2.as<float>();
                 mp.sg = c->sg2.as<unsigned>();
                 mp.bt = c->bt2.as<unsigned long long>();
                 mp.strip = c->strip2.as<float>();
-                mp.err = c->maperr.as<int>();
-                CBP_CUDA(cudaMemsetAsync(c->maperr.p, 0, sizeof(int), c->stream));
+                mp.err = maperr;
                 CBP_CUDA(cudaEventRecord(c->ev[6], c->stream));
                 launch_map(mp, c->stream);
                 CBP_CUDA(cudaEventRecord(c->ev[7], c->stream));
@@ -1162,78 +1168,62 @@ void process_queries(cbp_context* c, size_t nq, const size_t* qlens, char* const
             }
             r.last_npos2 = npos2;
             // sort keys of this slab's records, for the hit order
-            c->launches += launch_hit_keys(c->hitrecs.as<float>(), np, r.logE_thld, r.base_npass,
-                                           c->hitkeys.as<uint64_t>() + k * keycap, c->hitcnt.as<int>() + k,
-                                           c->stream);
+            c->launches += launch_hit_keys(hitrecs, np, r.logE_thld, r.base_npass,
+                                           keys_d, c->hitcnt.as<int>() + k, c->stream);
             c->stage_launches[5] += 1;
             // the results of the one slab are complete: the hit order too
-            const bool one = slabs.size() == 1;
             if (one) {
                 CBP_CUDA(cudaEventRecord(c->ev[8], c->stream));
-                const int nl = launch_hit_sort(c->hitkeys.as<uint64_t>() + k * keycap, np, c->stream);
+                const int nl = launch_hit_sort(keys_d, np, c->stream);
                 CBP_CUDA(cudaEventRecord(c->ev[9], c->stream));
                 c->launches += nl;
                 c->stage_launches[5] += nl;
             }
             const size_t off = r.h_recs.size();
-            const size_t recbytes = (size_t)np * kRecFloats * sizeof(float);
             r.h_recs.resize(off + (size_t)np * kRecFloats);
             // this slab's alignment rows go to the running offset of
             // the whole result (slot of pair K at newDst + K*Lq)
             const long long shift = r.base_len + r.base_npass * (long long)Lq;
             const long long slablen = npos2 + (long long)np * Lq;
-            for (int row = 0; row < 5; row++) r.h_alns[row].resize((size_t)(shift + slablen), 0);
-            // staged: flags, keys, records, rows
-            const size_t keybytes = one ? (size_t)np * sizeof(uint64_t) : 0;
-            const size_t small = 16 + keybytes + recbytes;
-            const bool staged = small + 5 * (size_t)slablen <= kMaxStaged;
-            c->rpin.reserve(16 + (staged ? small + 5 * (size_t)slablen : 0));
-            char* const pin = c->rpin.as<char>();
-            int* const pflags = reinterpret_cast<int*>(pin);
-            pflags[0] = pflags[1] = 0;
-            if (c->opt.mapaln)
-                CBP_CUDA(cudaMemcpyAsync(pflags, c->maperr.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-            if (one)
-                CBP_CUDA(cudaMemcpyAsync(pflags + 1, c->hitcnt.as<int>() + k, sizeof(int), cudaMemcpyDeviceToHost,
-                                         c->stream));
-            std::vector<uint64_t> keys;
-            if (staged) {
-                if (one)
-                    CBP_CUDA(cudaMemcpyAsync(pin + 16, c->hitkeys.as<uint64_t>() + k * keycap, keybytes,
-                                             cudaMemcpyDeviceToHost, c->stream));
-                CBP_CUDA(cudaMemcpyAsync(pin + 16 + keybytes, c->hitrecs.p, recbytes, cudaMemcpyDeviceToHost,
-                                         c->stream));
-                CBP_CUDA(cudaMemcpy2DAsync(pin + small, (size_t)slablen, c->alnbuf.p, (size_t)alnstride,
-                                           (size_t)slablen, 5, cudaMemcpyDeviceToHost, c->stream));
+            // records, flag and rows come down as they lie, with one slab the
+            // keys too and the rows stay there; large ones of several slabs go
+            // straight to their places
+            const size_t bytes = one ? keysoff + (size_t)np * sizeof(uint64_t) : keysoff;
+            const bool packed = one || bytes <= kMaxPacked;
+            if (!one)
+                for (int row = 0; row < 5; row++) r.h_alns[row].resize((size_t)(shift + slablen), 0);
+            if (packed) {
+                if (r.h_block.size() < bytes) r.h_block.resize(bytes);
+                CBP_CUDA(cudaMemcpyAsync(r.h_block.data(), c->results.p, bytes, cudaMemcpyDeviceToHost, c->stream));
             } else {
-                keys.resize(one ? (size_t)np : 0);
-                if (one)
-                    CBP_CUDA(cudaMemcpyAsync(keys.data(), c->hitkeys.as<uint64_t>() + k * keycap, keybytes,
-                                             cudaMemcpyDeviceToHost, c->stream));
-                CBP_CUDA(cudaMemcpyAsync(r.h_recs.data() + off, c->hitrecs.p, recbytes, cudaMemcpyDeviceToHost,
-                                         c->stream));
+                CBP_CUDA(cudaMemcpyAsync(&c->h_maperr, maperr, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+                CBP_CUDA(cudaMemcpyAsync(r.h_recs.data() + off, hitrecs, recbytes, cudaMemcpyDeviceToHost, c->stream));
                 for (int row = 0; row < 5; row++)
-                    CBP_CUDA(cudaMemcpyAsync(r.h_alns[row].data() + shift, c->alnbuf.as<char>() + (size_t)row * alnstride,
+                    CBP_CUDA(cudaMemcpyAsync(r.h_alns[row].data() + shift, alnbuf + (size_t)row * alnstride,
                                              (size_t)slablen, cudaMemcpyDeviceToHost, c->stream));
             }
             CBP_CUDA(cudaStreamSynchronize(c->stream));
-            c->h_maperr = pflags[0];
-            if (c->opt.mapaln && c->h_maperr)
-                throw Error(CBP_ERR_CUDA, "MAP realignment: a wait between the warps of a pair timed out");
-            if (staged) {
-                std::memcpy(r.h_recs.data() + off, pin + 16 + keybytes, recbytes);
-                for (int row = 0; row < 5; row++)
-                    std::memcpy(r.h_alns[row].data() + shift, pin + small + (size_t)row * slablen, (size_t)slablen);
+            if (packed) {
+                std::memcpy(&c->h_maperr, r.h_block.data() + flagoff, sizeof(int));
+                std::memcpy(r.h_recs.data() + off, r.h_block.data(), recbytes);
             }
             if (one) {
-                const int nrep = pflags[1];
-                if (nrep < 0 || nrep > np) throw Error(CBP_ERR_CUDA, "hit order: inconsistent count");
-                const uint64_t* kp = staged ? reinterpret_cast<const uint64_t*>(pin + 16) : keys.data();
-                r.h_order.resize((size_t)nrep);
-                for (int i = 0; i < nrep; i++) r.h_order[i] = (int32_t)(uint32_t)kp[i];
+                r.one_slab = true;
+                r.block_rows = rowsoff;
+                r.block_stride = (size_t)alnstride;
+                r.block_len = (size_t)slablen;
+                // the keys of the reported records, in order, come first
+                const uint64_t* keys = reinterpret_cast<const uint64_t*>(r.h_block.data() + keysoff);
+                for (int i = 0; i < np && keys[i] != kNotReported; i++) r.h_order.push_back((int32_t)(uint32_t)keys[i]);
                 CBP_CUDA(cudaEventElapsedTime(&ms, c->ev[8], c->ev[9]));
                 c->stage_ms[5] += ms;
+            } else if (packed) {
+                for (int row = 0; row < 5; row++)
+                    std::memcpy(r.h_alns[row].data() + shift, r.h_block.data() + rowsoff + (size_t)row * alnstride,
+                                (size_t)slablen);
             }
+            if (c->opt.mapaln && c->h_maperr)
+                throw Error(CBP_ERR_CUDA, "MAP realignment: a wait between the warps of a pair timed out");
             CBP_CUDA(cudaEventElapsedTime(&ms, c->ev[4], c->ev[5]));
             c->stage_ms[3] += ms;
             CBP_CUDA(cudaEventElapsedTime(&ms, c->ev[6], c->ev[7]));
@@ -1254,7 +1244,7 @@ void process_queries(cbp_context* c, size_t nq, const size_t* qlens, char* const
     // over the keys of all its records; the reported ones come first
     for (size_t k = 0; k < nq; k++) {
         QueryResult& r = res[k];
-        if (r.base_npass <= 0 || slabs.size() == 1) continue;   // one slab: done with its results
+        if (r.base_npass <= 0 || one) continue;   // one slab: done with its results
         uint64_t* keys_d = c->hitkeys.as<uint64_t>() + k * keycap;
         CBP_CUDA(cudaEventRecord(c->ev[4], c->stream));
         const int nl = launch_hit_sort(keys_d, r.base_npass, c->stream);
@@ -1368,14 +1358,13 @@ int cbp_destroy(cbp_context* c)
     c->query.release();
     if (c->phase1_exec) cudaGraphExecDestroy(c->phase1_exec);
     for (DevBuf* b : {&c->scores, &c->modscores, &c->btck, &c->bandbuf, &c->colorder, &c->dpmax, &c->dpcoords,
-                      &c->dprecs, &c->passidx, &c->passdst, &c->passcnt, &c->hitrecs, &c->nnweights,
-                      &c->cs2, &c->fb2, &c->sg2, &c->bt2, &c->strip2, &c->maperr, &c->alnbuf,
-                      &c->cvsmap, &c->statrecs, &c->dp1err, &c->hitkeys, &c->hitcnt, &c->fits, &c->qtrn})
+                      &c->dprecs, &c->passidx, &c->passdst, &c->passcnt, &c->results, &c->nnweights,
+                      &c->cs2, &c->fb2, &c->sg2, &c->bt2, &c->strip2,
+                      &c->cvsmap, &c->statrecs, &c->hitkeys, &c->hitcnt, &c->fits, &c->qtrn})
         b->release();
     c->sstab.release();
     c->dmstab.release();
     for (DevBuf* b : {&c->tcq, &c->tcerr}) b->release();
-    for (PinBuf* b : {&c->qpin, &c->cpin, &c->rpin}) b->release();
     for (auto& e : c->ev)
         if (e) cudaEventDestroy(e);
     if (c->stream) cudaStreamDestroy(c->stream);
@@ -1487,8 +1476,8 @@ int cbp_get_capacities(cbp_context* c, size_t query_len, size_t expected_profile
         size_t held_working = 0;
         for (const DevBuf* b : {&c->scores, &c->modscores, &c->btck, &c->bandbuf, &c->dpmax,
                                 &c->dpcoords, &c->dprecs, &c->passidx, &c->passdst, &c->passcnt,
-                                &c->hitrecs, &c->statrecs, &c->cs2, &c->fb2, &c->sg2, &c->bt2,
-                                &c->strip2, &c->maperr, &c->alnbuf})
+                                &c->results, &c->statrecs, &c->cs2, &c->fb2, &c->sg2, &c->bt2,
+                                &c->strip2})
             held_working += b->bytes;
         const size_t held_chunk = (c->db.use_count() == 1) ? c->db->bytes() : 0;
         const size_t still = c->mem_budget > held_working ? c->mem_budget - held_working : 0;
@@ -1733,11 +1722,11 @@ int cbp_get_alignments(cbp_context* c, char* rows, size_t row_stride, size_t* le
     return guarded([&] {
         check_ctx(c);
         const QueryResult& q = cur_result(c);
-        const size_t n = q.h_alns[0].size();
+        const size_t n = q.row_length();
         if (length) *length = n;
         if (rows) {
             if (row_stride < n) throw Error(CBP_ERR_ARG, "row stride smaller than the alignment rows");
-            for (int r = 0; r < 5; r++) std::memcpy(rows + (size_t)r * row_stride, q.h_alns[r].data(), n);
+            for (int r = 0; r < 5; r++) std::memcpy(rows + (size_t)r * row_stride, q.row(r), n);
         }
     });
 }
@@ -1751,10 +1740,10 @@ int cbp_format_hits(cbp_context* c, const cbp_format_options* fo, const char* co
         if (!c->have_db) throw Error(CBP_ERR_STATE, "no database chunk transferred");
         const ProfilesStore& db = *c->db;
         const QueryResult& q = cur_result(c);
-        const size_t n = q.h_alns[0].size();
+        const size_t n = q.row_length();
         std::vector<char> rows(5 * n);
         for (int r = 0; r < 5; r++)
-            if (n) std::memcpy(rows.data() + (size_t)r * n, q.h_alns[r].data(), n);
+            if (n) std::memcpy(rows.data() + (size_t)r * n, q.row(r), n);
         const int qss = c->query.h_ss.empty() ? 1 : c->query.h_ss[c->cur];
         rc = format_hits_from(q.h_recs.data(), q.h_recs.size() / kRecFloats, q.h_order.data(),
                               q.h_order.size(), rows.data(), n, n,

@@ -24,7 +24,6 @@ namespace {
 
 constexpr int kSortBlock = 4096;      // keys sorted in shared memory by one block
 constexpr int kSortThreads = 1024;
-constexpr uint64_t kNotReported = ~0ull;
 
 // an unsigned integer of the same order as the float (-0 taken as +0)
 __device__ __forceinline__ uint32_t ordered_bits(float f)

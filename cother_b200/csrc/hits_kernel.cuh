@@ -6,9 +6,11 @@
 
 namespace cbp {
 
+constexpr uint64_t kNotReported = ~0ull;   // the key of a record that is not reported
+
 // Keys of records base .. base+n-1 (`recs` holds the n records): the log
 // E-value's order in the high word and the record index in the low word for
-// a reported record (log E at most `logethld`, realigned), all ones
+// a reported record (log E at most `logethld`, realigned), kNotReported
 // otherwise; *nreported is increased by the reported count. Returns the
 // launches made.
 int launch_hit_keys(const float* recs, int n, float logethld, long long base, uint64_t* keys, int* nreported,
