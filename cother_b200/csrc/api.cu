@@ -184,21 +184,22 @@ using namespace cbp;
 namespace cbp {
 // Kernel variants for one query-length bin: rows per block of the score
 // kernel, the column-ordering window, warps per block of the phase-1 DP;
-// and, once tuned, each candidate's time on the sample.
+// and, once tuned, each candidate's time on the sample. The score kernel and
+// the DP are tuned apart, each by the first slab whose launches depend on it.
 constexpr int kScoreCandidates = 5;
 constexpr int kDpCandidates = 2;
 constexpr int kScoreRowsCand[kScoreCandidates] = {16, 8, 32, 16, 16};
 constexpr int kWindowCand[kScoreCandidates] = {1024, 1024, 1024, 256, 4096};
 constexpr int kDpWarpsCand[kDpCandidates] = {2, 1};
 constexpr int kPreferredScoreCand = 0;     // 16 rows, window 1,024
+constexpr int kPreferredDpCand = 1;        // 1 warp
 constexpr long long kTuneCells = 1 << 20;  // cells of a sample
 constexpr float kTuneMargin = 0.015f;      // a candidate must be this much faster to replace it
 struct Tuning {
     int rows = 16, window = kOrderWindow, dp_warps = 2;
-    bool tuned = false;
+    bool score_tuned = false, dp_tuned = false;
     float score_ms[kScoreCandidates] = {};
     float dp_ms[kDpCandidates] = {};
-    long long sample_cols = 0;
 };
 // The results of one query of a cbp_process or cbp_process_batch call.
 struct QueryResult {
@@ -617,17 +618,25 @@ std::vector<Slab> plan_slabs(const cbp_context* c, int Lq)
     return out;
 }
 
-// The tuner: on the first slab of a query-length bin, time each candidate
-// kernel variant on a sample of the slab (its first profiles, up to 32,768
-// positions and about a million cells, all query rows) and keep the fastest. A
-// million cells are two waves of the score kernel's blocks; the twelve timed
-// launches on them take about as long as searching 12 million cells, where
-// 32,768 positions made a first search against 200,000 positions four times as
-// long as the next. Every variant computes
-// the same cells, so the choice changes the time, never a result; the
-// sample's outputs are overwritten by the slab's own launches.
-void tune_kernels(cbp_context* c, const ScoreArgs& base, int p0, int p1, Tuning& t)
+// The tuner: on the first slab of a query-length bin whose launches depend on
+// the choice, time each candidate kernel variant on a sample of the slab (its
+// first profiles, up to 32,768 positions and about a million cells, all query
+// rows) and keep the fastest. A million cells are two waves of the score
+// kernel's blocks; the ten timed launches on them and those of the DP take
+// about as long as searching 12 million cells, where 32,768 positions made a
+// first search against 200,000 positions four times as long as the next. Every
+// variant computes the same cells, so the choice changes the time, never a
+// result; the sample's outputs are overwritten by the slab's own launches.
+//
+// dp: the DP of one query of the slab. With `apart` its launch for the maxima
+// gives every warp a profile of its own, and the candidates are timed in that
+// form whatever the sample's size; otherwise warps share a profile, the
+// candidates are one and the same launch, and its time stands for both.
+void tune_kernels(cbp_context* c, const ScoreArgs& base, const Dp1Args& dp, bool apart, int p0, int p1, Tuning& t)
 {
+    const bool score = !t.score_tuned && !score_plain(base);
+    const bool dpt = !t.dp_tuned && (apart || !(t.dp_ms[0] > 0.0f));
+    if (!score && !dpt) return;
     const ProfilesStore& db = *c->db;
     int pe = p0;
     long long ncols = 0;
@@ -652,7 +661,7 @@ void tune_kernels(cbp_context* c, const ScoreArgs& base, int p0, int p1, Tuning&
         return best;
     };
     int bs = 0;
-    for (int k = 0; k < kScoreCandidates; k++) {
+    for (int k = 0; score && k < kScoreCandidates; k++) {
         a.rows = kScoreRowsCand[k];
         t.score_ms[k] = time_it([&] {
             if (a.colorder)
@@ -669,37 +678,40 @@ void tune_kernels(cbp_context* c, const ScoreArgs& base, int p0, int p1, Tuning&
     // whose query lists take 42 KB), with half the re-reads of the database
     // lists. q400 x 1,000 profiles: 77.4 ms with 8 rows, 78.0 with 16, and 82
     // with 32.
-    if (t.score_ms[bs] > (1.0f - kTuneMargin) * t.score_ms[kPreferredScoreCand]) bs = kPreferredScoreCand;
-    Dp1Args d;
-    d.scores = a.scores;
+    if (score) {
+        if (t.score_ms[bs] > (1.0f - kTuneMargin) * t.score_ms[kPreferredScoreCand]) bs = kPreferredScoreCand;
+        t.rows = kScoreRowsCand[bs];
+        t.window = kWindowCand[bs];
+        t.score_tuned = true;
+    }
+    if (!dpt) return;
+    Dp1Args d = dp;
     d.ld = a.ld;
-    d.Lq = a.Lq;
-    d.qtrn = c->query.view.trn;
-    d.db = db.view;
-    d.col0 = a.col0;
-    d.p0 = p0;
     d.nprof = pe - p0;
-    d.btck = c->btck.as<uint8_t>();
-    d.bandbuf = c->bandbuf.as<float>();
-    d.maxsc = c->dpmax.as<float>();
-    d.maxcoords = c->dpcoords.as<uint32_t>();
-    d.recs = c->dprecs.as<Dp1Rec>();
+    d.order = nullptr;
+    d.apart = apart;
     // timed as the search runs it: the launch without backtrack codes over
     // every profile, then the codes launch, here with no candidate
     d.code_thld = INFINITY;
-    int bd = 0;
-    for (int k = 0; k < kDpCandidates; k++) {
+    for (int k = 0; k < (apart ? kDpCandidates : 1); k++) {
         d.warps = kDpWarpsCand[k];
         int nl = 0;
         t.dp_ms[k] = time_it([&] { nl = launch_dp1(d, c->stream); });
         c->launches += 2 * (uint64_t)nl;   // two timed repetitions
-        if (t.dp_ms[k] < t.dp_ms[bd]) bd = k;
     }
-    t.rows = kScoreRowsCand[bs];
-    t.window = kWindowCand[bs];
+    if (!apart) {
+        std::fill(t.dp_ms + 1, t.dp_ms + kDpCandidates, t.dp_ms[0]);
+        return;
+    }
+    // One warp to a block is 13 to 16 % faster on 10,000 and more profiles of
+    // all query lengths (400 x 20,000: 7.33 ms against 8.46), so another value
+    // must be faster by more than the sample's noise.
+    int bd = 0;
+    for (int k = 1; k < kDpCandidates; k++)
+        if (t.dp_ms[k] < t.dp_ms[bd]) bd = k;
+    if (t.dp_ms[bd] > (1.0f - kTuneMargin) * t.dp_ms[kPreferredDpCand]) bd = kPreferredDpCand;
     t.dp_warps = kDpWarpsCand[bd];
-    t.sample_cols = ncols;
-    t.tuned = true;
+    t.dp_tuned = true;
 }
 
 }  // namespace
@@ -893,9 +905,38 @@ void process_queries(cbp_context* c, size_t nq, const size_t* qlens, char* const
         // the column order only balances the DDMS loops of a warp's lanes;
         // without that term the identity keeps the stores coalesced
         a.colorder = a.ddmswgt > 0.0f ? c->colorder.as<int>() : nullptr;
+        std::vector<Dp1Args> d(nq);
+        for (size_t k = 0; k < nq; k++) {
+            const QueryResult& r = res[k];
+            d[k].scores = a.scores + (long long)r.row0 * a.ld;
+            d[k].ld = a.ld;
+            d[k].Lq = r.Lq;
+            d[k].qtrn = qtrn[k];
+            d[k].db = c->db->view;
+            d[k].col0 = s.col0;
+            d[k].p0 = s.p0;
+            d[k].nprof = s.p1 - s.p0;
+            // one slab of the whole chunk takes its profiles longest first
+            d[k].order = d[k].nprof == c->db->view.P ? c->db->view.order : nullptr;
+            d[k].btck = c->btck.as<uint8_t>() + (long long)r.row0 * a.ld;
+            d[k].bandbuf = c->bandbuf.as<float>();
+            d[k].maxsc = c->dpmax.as<float>() + k * maxprof;
+            d[k].maxcoords = c->dpcoords.as<uint32_t>() + k * maxprof;
+            // codes for the finalization's candidates only, unless all are asked for
+            d[k].code_thld = c->opt.all_codes ? -INFINITY : r.score_thld;
+            d[k].recs = c->dprecs.as<Dp1Rec>() + k * maxprof;
+            d[k].err = dp1err;
+        }
+
         Tuning& tn = c->tuning[Ltot / 64];
-        if (c->opt.autotune && !tn.tuned) tune_kernels(c, a, s.p0, s.p1, tn);
+        if (c->opt.autotune) {
+            // the DP's sample: a query whose warps sweep a profile each, if there is one
+            size_t kd = 0;
+            while (kd + 1 < nq && dp1_profile_warps(d[kd].nprof, d[kd].Lq) > 1) kd++;
+            tune_kernels(c, a, d[kd], dp1_profile_warps(d[kd].nprof, d[kd].Lq) == 1, s.p0, s.p1, tn);
+        }
         a.rows = tn.rows;
+        for (Dp1Args& x : d) x.warps = tn.dp_warps;
         if (tc) {
             // the profile-profile sums on the tensor cores, per query (its
             // database operand depends on the query's background)
@@ -926,29 +967,6 @@ void process_queries(cbp_context* c, size_t nq, const size_t* qlens, char* const
             a.dots_in_scores = true;
         }
 
-        std::vector<Dp1Args> d(nq);
-        for (size_t k = 0; k < nq; k++) {
-            const QueryResult& r = res[k];
-            d[k].scores = a.scores + (long long)r.row0 * a.ld;
-            d[k].ld = a.ld;
-            d[k].Lq = r.Lq;
-            d[k].qtrn = qtrn[k];
-            d[k].db = c->db->view;
-            d[k].col0 = s.col0;
-            d[k].p0 = s.p0;
-            d[k].nprof = s.p1 - s.p0;
-            // one slab of the whole chunk takes its profiles longest first
-            d[k].order = d[k].nprof == c->db->view.P ? c->db->view.order : nullptr;
-            d[k].btck = c->btck.as<uint8_t>() + (long long)r.row0 * a.ld;
-            d[k].bandbuf = c->bandbuf.as<float>();
-            d[k].maxsc = c->dpmax.as<float>() + k * maxprof;
-            d[k].maxcoords = c->dpcoords.as<uint32_t>() + k * maxprof;
-            // codes for the finalization's candidates only, unless all are asked for
-            d[k].code_thld = c->opt.all_codes ? -INFINITY : r.score_thld;
-            d[k].recs = c->dprecs.as<Dp1Rec>() + k * maxprof;
-            d[k].warps = tn.dp_warps;
-            d[k].err = dp1err;
-        }
         auto pass_idx = [&](size_t k) { return c->passidx.as<int>() + k * maxprof; };
         auto pass_dst = [&](size_t k) { return c->passdst.as<long long>() + k * maxprof; };
         auto pass_cnt = [&](size_t k) { return reinterpret_cast<int*>(c->passcnt.as<char>() + 16 * k); };
@@ -1825,7 +1843,7 @@ int cbp_set_kernels(cbp_context* c, size_t query_len, int rows, int window, int 
         t.rows = rows;
         t.window = window;
         t.dp_warps = dp_warps;
-        t.tuned = true;
+        t.score_tuned = t.dp_tuned = true;
     });
 }
 

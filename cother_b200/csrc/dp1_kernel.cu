@@ -842,7 +842,7 @@ void launch_dp1_pass(const Dp1Args& a, bool bulk, cudaStream_t stream)
     // a codes launch behind one for the maxima sweeps the candidates alone,
     // about 1 % of a large database: at most an eighth is allowed for
     const int work = kCodes && a.code_thld != -INFINITY ? (a.nprof + 7) / 8 : a.nprof;
-    const int share = bulk ? dp1_profile_warps(work, a.Lq) : 1;
+    const int share = bulk && !a.apart ? dp1_profile_warps(work, a.Lq) : 1;
     switch (share) {
     case 8: launch_dp1_variant<8, true, true, kCodes>(a, stream); return;
     case 4: launch_dp1_variant<4, true, true, kCodes>(a, stream); return;

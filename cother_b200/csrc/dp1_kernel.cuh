@@ -33,6 +33,7 @@ struct Dp1Args {
     uint32_t* maxcoords = nullptr;   // [nprof]
     Dp1Rec* recs = nullptr;          // [nprof]
     int warps = 2;                   // warps per block where each sweeps a profile of its own: 1 or 2
+    bool apart = false;              // each does, whatever dp1_profile_warps() says
     // the order the launches take the slab's profiles in, [nprof] (longest
     // first, so that no long one is left for the end); null: as they come
     const int* order = nullptr;

@@ -778,6 +778,11 @@ void launch_column_order(const uint8_t* dstlen, long long col0, int ncols, long 
     CBP_CHECK_LAUNCH();
 }
 
+bool score_plain(const ScoreArgs& a)
+{
+    return a.q.P == 1 && !(a.ddmswgt > 0.0f) && !(a.cvswgt > 0.0f) && !a.colorder;
+}
+
 template <int kRows, bool kStacked>
 void launch_score_rows(const ScoreArgs& a, cudaStream_t stream)
 {
@@ -786,7 +791,7 @@ void launch_score_rows(const ScoreArgs& a, cudaStream_t stream)
         a.cvswgt > 0.0f ? sizeof(float) * ((kNCV + 2) * kCols + kRows * (kNCV + 1) + 2 * kRows) : 0;
     if (a.ddmswgt > 0.0f) {
         score_matrix_kernel<kRows, kStacked, true><<<grid, kThreads, cvs_smem, stream>>>(a);
-    } else if (!kStacked && !(a.cvswgt > 0.0f) && !a.colorder) {
+    } else if (score_plain(a)) {
         const dim3 pgrid((unsigned)ceil_div(a.ncols, kPlainCols), (unsigned)ceil_div(a.Lq, kPlainRows));
         if (a.dots_in_scores) score_plain_kernel<true><<<pgrid, kPlainCols, 0, stream>>>(a);
         else score_plain_kernel<false><<<pgrid, kPlainCols, 0, stream>>>(a);

@@ -45,6 +45,9 @@ constexpr int kOrderWindow = 1024;
 constexpr int kMaxOrderWindow = 4096;
 
 void launch_score_matrix(const ScoreArgs& a, cudaStream_t stream);
+// Whether the launch runs the kernel without the distance and context-vector
+// terms, whose blocks are of one size (ScoreArgs::rows has no effect).
+bool score_plain(const ScoreArgs& a);
 // Fill order[0..ld) for the slab columns [col0, col0+ncols): within each
 // window of `window` slots (a multiple of 32, at most kMaxOrderWindow), the
 // window's columns by descending distance list length; slots past ncols

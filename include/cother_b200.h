@@ -594,7 +594,12 @@ int cbp_set_max_slab_positions(cbp_context* ctx, size_t max_positions);
  * autotune = 0): score-kernel query rows per block, column-ordering window,
  * phase-1 DP warps per block; and in ms[0..n) the tuned candidates' times on
  * the sample (score variants (16,1024), (8,1024), (32,1024), (16,256),
- * (16,4096), then DP variants 2 and 1 warps). */
+ * (16,4096), then DP variants 2 and 1 warps). A choice is made by the first
+ * search that depends on it. The score variants do not matter to a search of
+ * one query with DDMSWGT = CVSWGT = 0 (their times stay 0), nor the DP's warps
+ * per block where the warps of a block share a profile (slabs of up to 9,472
+ * profiles for queries of more than 64 positions): both DP times are then
+ * that launch's, and dp_warps stays 2 until a larger slab comes. */
 int cbp_get_tuning(cbp_context* ctx, size_t query_len, int* rows, int* window, int* dp_warps,
                    float* ms, int n);
 
