@@ -191,9 +191,11 @@ constexpr int kDpCandidates = 2;
 constexpr int kScoreRowsCand[kScoreCandidates] = {16, 8, 32, 16, 16};
 constexpr int kWindowCand[kScoreCandidates] = {1024, 1024, 1024, 256, 4096};
 constexpr int kDpWarpsCand[kDpCandidates] = {2, 1};
-constexpr int kPreferredScoreCand = 0;     // 16 rows, window 1,024
+constexpr int kPreferredDdmsCand = 1;      // 8 rows, window 1,024: with the distance term
+constexpr int kPreferredPlainCand = 2;     // 32 rows: without it
 constexpr int kPreferredDpCand = 1;        // 1 warp
 constexpr long long kTuneCells = 1 << 20;  // cells of a sample
+constexpr long long kTunePlainCells = 8 << 20;   // without the distance term
 constexpr float kTuneMargin = 0.015f;      // a candidate must be this much faster to replace it
 struct Tuning {
     int rows = 16, window = kOrderWindow, dp_warps = 2;
@@ -624,7 +626,9 @@ std::vector<Slab> plan_slabs(const cbp_context* c, int Lq)
 // rows) and keep the fastest. A million cells are two waves of the score
 // kernel's blocks; the ten timed launches on them and those of the DP take
 // about as long as searching 12 million cells, where 32,768 positions made a
-// first search against 200,000 positions four times as long as the next. Every
+// first search against 200,000 positions four times as long as the next.
+// Without the distance term a cell takes a thirtieth of the time, and on one
+// or two waves 16 rows a block look as fast as 32: eight million cells. Every
 // variant computes the same cells, so the choice changes the time, never a
 // result; the sample's outputs are overwritten by the slab's own launches.
 //
@@ -640,7 +644,8 @@ void tune_kernels(cbp_context* c, const ScoreArgs& base, const Dp1Args& dp, bool
     const ProfilesStore& db = *c->db;
     int pe = p0;
     long long ncols = 0;
-    const long long most = std::min<long long>(32768, std::max<long long>(1024, kTuneCells / base.Lq));
+    const long long cells = base.ddmswgt > 0.0f ? kTuneCells : kTunePlainCells;
+    const long long most = std::min<long long>(32768, std::max<long long>(1024, cells / base.Lq));
     while (pe < p1 && (pe == p0 || ncols + db.h_plen[pe] <= most)) ncols += db.h_plen[pe++];
     ScoreArgs a = base;
     a.ncols = (int)ncols;
@@ -663,23 +668,30 @@ void tune_kernels(cbp_context* c, const ScoreArgs& base, const Dp1Args& dp, bool
     int bs = 0;
     for (int k = 0; score && k < kScoreCandidates; k++) {
         a.rows = kScoreRowsCand[k];
+        if (!a.colorder && k > 0 && a.rows == kScoreRowsCand[0]) {   // the same launch: no column order
+            t.score_ms[k] = t.score_ms[0];
+            continue;
+        }
         t.score_ms[k] = time_it([&] {
             if (a.colorder)
                 launch_column_order(db.view.dstlen, a.col0, a.ncols, a.ld, kWindowCand[k], c->colorder.as<int>(),
                                     c->stream);
             launch_score_matrix(a, c->stream);
         });
-        c->launches += 4;
+        c->launches += a.colorder ? 4 : 2;
         if (t.score_ms[k] < t.score_ms[bs]) bs = k;
     }
-    // The candidates' sample times lie within about 1 % of each other, the
-    // sample's noise. Unless one is clearly faster, keep 16 rows per block
-    // with the default window: 8 blocks fit an SM as with 8 rows (5 with 32,
-    // whose query lists take 42 KB), with half the re-reads of the database
-    // lists. q400 x 1,000 profiles: 77.4 ms with 8 rows, 78.0 with 16, and 82
-    // with 32.
+    // Unless another is faster by more than the sample's noise, the variant
+    // that is the fastest on whole searches. With the distance term 8 rows a
+    // block (22 KB of shared memory: 8 blocks an SM, bound by registers; 7 with
+    // 16 rows, 5 with 32): score stage of 400 x 1,500 profiles 113.1 ms with
+    // 8, 114.7 with 16, 123.2 with 32; 64 x 3,000 19.6 / 19.8 / 21.5. Without
+    // it 32 rows, which read the database's fields the fewest times: 333 x
+    // 4,000 profiles with context vectors 11.1 / 7.9 / 6.7 ms, four stacked
+    // queries x 5,000 profiles 33.1 / 26.2 / 23.5.
     if (score) {
-        if (t.score_ms[bs] > (1.0f - kTuneMargin) * t.score_ms[kPreferredScoreCand]) bs = kPreferredScoreCand;
+        const int pref = base.ddmswgt > 0.0f ? kPreferredDdmsCand : kPreferredPlainCand;
+        if (t.score_ms[bs] > (1.0f - kTuneMargin) * t.score_ms[pref]) bs = pref;
         t.rows = kScoreRowsCand[bs];
         t.window = kWindowCand[bs];
         t.score_tuned = true;
