@@ -182,11 +182,13 @@ __device__ __forceinline__ float ddms_offer(DdmsReg& r, bool on, uint32_t pos, f
 // commutes exactly with IEEE rounding, so the sums are the reference's
 // times 2^-7, bit for bit. An odd element's mean 0.5*(a+b) is exact once a+b
 // is rounded, so adding it is one saturating fma(0.5, a+b, sum). The bits of
-// a sum, as an integer, are 0 when it is zero and above 105 x 2^22 (the bits
-// of 2^-75) when not: the table's values are multiples of 2^-56, and so is
-// every sum of them. So the number of elements since the last zero, in units
-// of 2^22, is min(c + 2^22, bits), one instruction (VIADDMNMX) for the two
-// that a float length needs.
+// a sum, as an integer, are 0 when it is zero and 158 x 2^22 (the bits of
+// 2^-48) at least when not: the scaled values are multiples of 2^-47 (checked
+// by build_dms_table()), their means of 2^-48, and so is every sum of them. A
+// length is 105 at most (a list holds 99 elements, and the last two steps end
+// up to six past it), so the number of elements since the last zero, in units of
+// 2^22, is min(c + 2^22, bits), one instruction (VIADDMNMX) for the two that a
+// float length needs.
 //
 // A step can offer a candidate (DSTSEGM >= 5) only when its first sum is
 // positive and c1 >= DSTSEGM - 3, which is all that every step tests; the
@@ -348,7 +350,7 @@ score_matrix_kernel(const ScoreArgs a)
     __shared__ int s_dlen[kCols];
     __shared__ int s_qlen[kRows];
     // context vectors and their log priors and squared norms (CVSWGT > 0):
-    // dynamic shared memory, absent otherwise, so that ten blocks fit an SM
+    // dynamic shared memory, absent otherwise, so that more blocks fit an SM
     extern __shared__ float s_cvsdyn[];
     float (*s_dcv)[kCols] = reinterpret_cast<float (*)[kCols]>(s_cvsdyn);
     float (*s_dcvpn)[kCols] = reinterpret_cast<float (*)[kCols]>(s_cvsdyn + kNCV * kCols);
@@ -838,6 +840,13 @@ void build_dms_table(float* T)
             volatile float slope = sl0 * inv;
             T[a1 * kDstCard + a2] = std::fmaf((float)d1, slope, intpt);
         }
+    // what ddms_diagonal() counts on: multiples of 2^-40 (times 2^-7 there), and
+    // no sum of a list's values above 1 after that scaling
+    for (int i = 0; i < kDstCard * kDstCard; i++) {
+        const float v = std::ldexp(T[i], 40);
+        if (v != std::rint(v) || !(T[i] <= 1.0f))
+            throw Error(CBP_ERR_ARG, "distance pair scores: a value outside the kernel's range");
+    }
 }
 
 }  // namespace cbp
