@@ -33,23 +33,25 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 DEFAULT_WORKLOAD = "q400_db50k"
-# DRAM bytes (read + write) per cell of one score_matrix_kernel launch,
-# measured by ncu on q400 x 2,000 profiles (3.03 GB for 195.0 M cells with
-# the 32-row variant: 8 B/cell of score writes plus the database lists
-# re-read by each block of query rows); the traffic grows with the cells
-SCORE_DRAM_BYTES_PER_CELL = 15.51
+# DRAM bytes that one score_matrix_kernel launch reads per database position
+# and block of query rows when the database exceeds L2: 5.94 GB for 13 blocks
+# of 8 rows and 1,983,012 positions (ncu, one pass, 104 x 8,000 profiles; the
+# launch wrote 1.64 GB, 8 B/cell)
+SCORE_DRAM_READ_PER_POSITION = 230.0
 
 
 def score_traffic_per_cell(rows: int) -> float:
     """DRAM bytes per cell of the score kernel with `rows` query rows per
     block: the 8 B/cell of score writes plus the database reads, which each
-    block of rows repeats (measured at 32 rows)."""
-    return 8.0 + (SCORE_DRAM_BYTES_PER_CELL - 8.0) * 32.0 / rows
+    block of rows repeats."""
+    return 8.0 + SCORE_DRAM_READ_PER_POSITION / rows
 
 
 STAGES = ["score_matrix", "phase1_dp", "phase1_finalize", "statistics", "map_realignment", "hit_order"]
-OPS_PER_DDMS_STEP = 50  # algorithmic ops of one 4-cell DDMS step (2 pair scores,
-                        # 2 interpolations, 4 segment updates, 1 top-3 register)
+OPS_PER_DDMS_STEP = 50  # ops of one 4-cell DDMS step (2 pair scores, 2 interpolations,
+                        # 4 segment updates, 1 top-3 register offer), as the kernel performs
+                        # it (it issues 51 instructions a step): the fraction of the issue
+                        # rate says how busy the lanes are, not how few operations would do
 
 
 def parse():
@@ -523,10 +525,9 @@ def main():
                 "frac": achieved / alu_peak,
                 "traffic": score_traffic_per_cell(rows) * float(Lq) * Ndb,
                 "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one "
-                                  "score_matrix_kernel launch at q400 x 2,000 profiles with 32 "
-                                  "rows per block, scaled by cells and, for the %d-row variant "
-                                  "in use, by the database reads per block "
-                                  "(profiles/score_matrix_kernel_q400_db2k.md)" % rows,
+                                  "score_matrix_kernel launch at 104 x 8,000 profiles with 8 rows "
+                                  "per block, scaled by cells and by the database reads of each "
+                                  "block of %d rows" % rows,
                 "kernel": "score_matrix_kernel",
                 "peak_source": "148 SMs x 128 FP32 lanes x max SM clock (nominal issue rate)",
                 "hbm_bytes_per_launch": float(Lq) * Ndb * 8,

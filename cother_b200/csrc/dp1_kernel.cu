@@ -39,11 +39,11 @@ __device__ __forceinline__ int corner_edge(int Lq, int Ld)
     return e > 60 ? 60 : e;
 }
 
-// The band layout. A warp sweeps bands of 64 query rows, two per lane: lane t holds rows r0+2t (row "A") and r0+2t+1 (row
-// "B") and is at column s-t at step s. Row A takes its "up" states from
-// lane t-1's row B by shuffle, row B from the lane's own row A; so one
-// shuffle set, one read of the column's transitions and one ring index
-// serve two cells. The reference computes 32-row bands
+// The band layout. A warp sweeps bands of 64 query rows, two per lane: lane t
+// holds rows r0+2t (row "A") and r0+2t+1 (row "B") and is at column s-t at
+// step s. Row A takes its "up" states from lane t-1's row B by shuffle, row B
+// from the lane's own row A; so one shuffle set, one read of the column's
+// transitions and one ring index serve two cells. The reference computes 32-row bands
 // (src/libmycu/cudp/CuBatchDP_init_btck.cu:93-160); its band boundaries
 // only set the column -1 states of each row and the diagonal of a band's
 // last row at column 0, which are reproduced per row (row mod 32).

@@ -197,10 +197,11 @@ __device__ __forceinline__ float ddms_offer(DdmsReg& r, bool on, uint32_t pos, f
 // scheduler), with the ALU pipe, which takes an instruction every other
 // cycle, at 69 %: the steps' arithmetic is therefore spread over both pipes
 // (sums and masks FMA, lengths ALU, table offsets the FMA pipe's dp4a).
-// Measured at q400 x 1,000 profiles: 51.0 warp instructions a step and 77.4
-// ms, against 59.2 and 85.8 ms with float lengths, the masked sums in every
-// step and no threshold per segment; with the masks in every step 82 ms, with
-// a running maximum tested first 86 ms, with votes for the branches 91 ms.
+// Measured at q400 x 1,000 profiles, 16 rows a block: 51.0 warp instructions
+// a step and 77.4 ms, against 59.2 and 85.8 ms with float lengths, the masked
+// sums in every step and no threshold per segment; with the masks in every
+// step 82 ms, with a running maximum tested first 86 ms, with votes for the
+// branches 91 ms.
 //
 // qw: words of elements 1.. of the query list on this diagonal, q0 its
 // element 0; dw, sel: the words that hold elements 1.. of the database list
