@@ -264,7 +264,7 @@ struct cbp_context {
     DevBuf scores, modscores, btck, bandbuf, colorder, dpmax, dpcoords, dprecs, passidx, passdst, passcnt;
     DevBuf statrecs, cs2, fb2, sg2, bt2, strip2;
     DevBuf results;            // of the query in hand: hit records, the MAP stage's flag, alignment rows
-    DevBuf hitkeys, hitcnt;    // sort keys of all records of a query, reported count
+    DevBuf hitkeys, hitcnt;    // several slabs: sort keys of all records of a query; reported count
     DevBuf fits;               // the precision forms: FP64 and FP32 parameter fits per passed pair
     DevBuf qtrn;               // batches: each query's transitions as [7][Lq+1]
 
